@@ -293,7 +293,8 @@ def _run_scan(s, c):
 def _prepare_ros(s, c, g):
     s.clouds = []
     for k, (d, t, o) in enumerate(_lidar(g, c["n"], N_WARM + N_POSES)):
-        lost = ~torch.isfinite(t) | (torch.rand(c["n"], device=DEV, generator=g) < 0.01)
+        # a sensor that sees 100 m and drops one return in a hundred
+        lost = ~(t < 100.0) | (torch.rand(c["n"], device=DEV, generator=g) < 0.01)
         p = torch.where(lost[:, None], torch.full_like(d, math.nan), d * t[:, None])
         yaw = 0.02 * k  # the cloud in the frame of a sensor turned by yaw
         r = torch.tensor([[math.cos(yaw), -math.sin(yaw), 0], [math.sin(yaw), math.cos(yaw), 0],
