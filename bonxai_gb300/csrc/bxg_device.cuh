@@ -61,7 +61,7 @@ enum : int {
   C_CAST = 4,       // rays queued for the current scan
   C_FREE_LEAF = 5,  // entries on the leaf free stack
   C_LIST = 6,       // leaf blocks on the scan's marked list (bxg_mark.cuh)
-  C_TASK = 7,       // next block task of the mark phase
+  C_SEGS = 7,       // segments of the scan's rays (bxg_mark.cuh)
   C_STATS = 8,      // 64-bit statistics start here (pairs of words)
   C_WORDS = 32,
 };
@@ -443,6 +443,12 @@ __device__ __forceinline__ void axis_init(AxisStep& a, uint32_t d, uint32_t m, u
                                           float rtm, uint32_t k0, uint32_t W) {
   divmod_small(2u * k0 * d + m, two_m, rtm, a.n, a.r);
   divmod_small(2u * W * d, two_m, rtm, a.Q, a.R);
+}
+// (n, r) at cell k of a long ray.
+__device__ __forceinline__ void axis_start64(AxisStep& a, uint32_t d, uint32_t m, uint32_t k) {
+  const unsigned long long num = 2ull * k * d + m, two_m = 2ull * m;
+  a.n = static_cast<uint32_t>(num / two_m);
+  a.r = static_cast<uint32_t>(num % two_m);
 }
 __device__ __forceinline__ void axis_advance(AxisStep& a, uint32_t two_m) {
   a.n += a.Q;

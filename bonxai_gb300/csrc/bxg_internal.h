@@ -9,6 +9,7 @@
 
 #include "bonxai_gb300.h"
 #include "bxg_device.cuh"
+#include "bxg_mark.cuh"
 
 namespace bxg {
 
@@ -188,6 +189,9 @@ struct bxg_pmap_s {
   // between scans; sized for cube_blocks leaf blocks
   bxg::DevBuf cube_bits, cube_touch, cube_list;
   size_t cube_blocks = 0;
+  // root bits of the marked cells and the rays' segments, of the per-scan form
+  bxg::DevBuf cube_roots, ray_segs, ray_tails;
+  bool has_segs = false;  // the ray list's segments are in ray_segs, long rays in ray_tails
   cudaEvent_t ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
   ~bxg_pmap_s() {
     for (auto& e : ev)
@@ -196,8 +200,14 @@ struct bxg_pmap_s {
 };
 
 namespace bxg {
-struct LeafDir;
-struct RayCube;
+// The cube of a scan's ray phase from origin cell (ox, oy, oz) whose rays end
+// within `reach` (world units) of the origin; with `reach` unknown (0), infinite or above the
+// size limit, Q->open is set and the cube holds the rays' first Q->kin
+// cells. *ok = false when the scan cannot use one (other node sizes, non-finite
+// points kept, single pass asked for). rays: room for their segments (0: none).
+// Buffers grow here (cudaMalloc, zeroed).
+int scan_cube(bxg_pmap_s* pm, int ox, int oy, int oz, double reach, uint64_t rays, ScanCube* Q,
+              bool* ok);
 // The cube bitmap of a scan's ray phase from origin cell (ox, oy, oz) whose
 // rays end within `reach` (world units) of the origin: *ok = false when the
 // scan cannot use one (leaf_bits other than 3, non-finite points kept, a cube

@@ -15,14 +15,14 @@
 //   k_apply       only after a pool ran out: completes the listed endpoints.
 //   k_mark        the ray phase's first part: every listed ray's cells set
 //                 their bits in the scan's cube bitmap (bxg_mark.cuh).
-//   k_list_touched  the marked leaf blocks onto a list, in cube order.
-//   k_apply_rays  per listed leaf block, get-or-create the leaf and apply the
-//                 miss update to its marked cells.
-//   k_rays        the single-pass form of the ray phase, for scans the cube
-//                 does not cover (rays queued by addHitPoint/addMissPoint,
-//                 kept non-finite points, cubes above the size limit): a group
-//                 of W lanes walks one ray, W consecutive cells per step,
-//                 creating leaves on the way and applying the miss update.
+//   k_apply_rays  per marked leaf, get-or-create the leaf and apply the miss
+//                 update to its marked cells.
+//   k_tail        only when rays may be longer than the cube (no range limit,
+//                 queued rays): walks the rest of those that are.
+//   k_rays        the single-pass form of the ray phase, for maps that keep
+//                 non-finite points or ask for it: a group of W lanes walks one
+//                 ray, W consecutive cells per step, creating leaves on the way
+//                 and applying the miss update.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -38,9 +38,16 @@ namespace bxg {
 // zero: bit 0 -- the scan's statistics start at zero; bit 1 -- the ray list
 // starts empty (no rays queued by earlier addHitPoint/addMissPoint batches).
 // Done by the first kernel of a scan instead of memsets.
-enum : int { ZERO_STATS = 1, ZERO_CAST = 2 };
-__device__ __forceinline__ void zero_scan_stats(const DMap& M, int zero) {
+// bit 2 -- the ray phase's root bits and segment count start at zero.
+enum : int { ZERO_STATS = 1, ZERO_CAST = 2, ZERO_RAYS = 4 };
+__device__ __forceinline__ void zero_scan_stats(const DMap& M, int zero,
+                                                uint32_t* roots = nullptr,
+                                                uint32_t root_words = 0) {
+  for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < root_words;
+       t += gridDim.x * blockDim.x)
+    roots[t] = 0u;
   if (blockIdx.x != 0) return;
+  if ((zero & ZERO_RAYS) && threadIdx.x == 33) M.ctr[C_SEGS] = M.ctr[C_LIST] = 0u;
   if ((zero & ZERO_STATS) && threadIdx.x < S_COUNT)
     reinterpret_cast<unsigned long long*>(M.ctr + C_STATS)[threadIdx.x] = 0ull;
   if ((zero & ZERO_CAST) && threadIdx.x == 32) M.ctr[C_CAST] = 0u;
@@ -50,8 +57,9 @@ template <typename PT>
 __global__ void k_endpoints(const __grid_constant__ DMap M, const uint8_t* __restrict__ pts, size_t stride, uint32_t n,
                             double fx, double fy, double fz, double max_range, double mr2,
                             double inv_res, int keep_nonfinite, int4* __restrict__ ep,
-                            uint4* tab, uint32_t tmask, int zero_stats, EpFast F) {
-  zero_scan_stats(M, zero_stats);
+                            uint4* tab, uint32_t tmask, int zero_stats, EpFast F,
+                            uint32_t* roots, uint32_t root_words) {
+  zero_scan_stats(M, zero_stats, roots, root_words);
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   int4 e = make_int4(0, 0, 0, EP_SKIP);
   if (i < n) {
@@ -92,8 +100,9 @@ __global__ void k_endpoints_sensor(const __grid_constant__ DMap M, const uint8_t
                                    uint32_t n, Xf xf, double fx, double fy, double fz,
                                    double max_range, double mr2, double inv_res,
                                    int4* __restrict__ ep, uint4* tab, uint32_t tmask,
-                                   int zero_stats, EpFast F) {
-  zero_scan_stats(M, zero_stats);
+                                   int zero_stats, EpFast F, uint32_t* roots,
+                                   uint32_t root_words) {
+  zero_scan_stats(M, zero_stats, roots, root_words);
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float* p = reinterpret_cast<const float*>(pts + size_t(i) * stride);
@@ -130,8 +139,9 @@ __global__ void k_endpoints_kind(const __grid_constant__ DMap M, const double* _
 // lengths (a per-warp atomic on three shared counters serialised in L2).
 __global__ void __launch_bounds__(256) k_winners(const __grid_constant__ DMap M, const int4* __restrict__ ep, uint32_t n,
                           const uint4* __restrict__ tab, uint32_t tmask, int ox, int oy, int oz,
-                          int32_t u, Opts o, int4* __restrict__ cast, uint32_t cast_cap) {
-  __shared__ uint32_t s_cnt[8], s_pts[8], s_base;
+                          int32_t u, Opts o, int4* __restrict__ cast, uint32_t cast_cap,
+                          const __grid_constant__ ScanCube Q) {
+  __shared__ uint32_t s_cnt[8], s_pts[8], s_base, s_seg[8], s_seg_base, s_tail[8], s_tail_base;
   __shared__ unsigned long long s_len[8];
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   bool add = false;
@@ -148,14 +158,27 @@ __global__ void __launch_bounds__(256) k_winners(const __grid_constant__ DMap M,
   const uint32_t len = add ? chebyshev(ox, oy, oz, e.x, e.y, e.z) : 0u;
   const unsigned long long wlen = __reduce_add_sync(0xffffffffu, len >> 16) * 65536ull +
                                   __reduce_add_sync(0xffffffffu, len & 0xFFFFu);
+  // with a cube, the ray's segments go on the scan's list of segments
+  const uint32_t nseg = add && Q.segs ? far_segments(Q, len) : 0u;
+  uint32_t seg = nseg;
+#pragma unroll
+  for (int o2 = 1; o2 < 32; o2 <<= 1) {
+    const uint32_t v = __shfl_up_sync(0xffffffffu, seg, o2);
+    if (lane >= unsigned(o2)) seg += v;
+  }
+  if (lane == 31) s_seg[wid] = seg;
+  // and the rays that leave the cube on the list of those
+  const unsigned tails =
+      __ballot_sync(0xffffffffu, add && Q.tails && len > Q.kin);
   if (lane == 0) {
     s_cnt[wid] = __popc(am);
+    s_tail[wid] = __popc(tails);
     s_pts[wid] = __popc(valid);
     s_len[wid] = wlen;
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    uint32_t tot = 0, pts = 0;
+    uint32_t tot = 0, pts = 0, segs = 0, tl_n = 0;
     unsigned long long tl = 0;
     for (unsigned w = 0; w < blockDim.x / 32; w++) {
       const uint32_t c = s_cnt[w];
@@ -163,19 +186,39 @@ __global__ void __launch_bounds__(256) k_winners(const __grid_constant__ DMap M,
       tot += c;
       pts += s_pts[w];
       tl += s_len[w];
+      const uint32_t g = s_seg[w];
+      s_seg[w] = segs;
+      segs += g;
+      const uint32_t r = s_tail[w];
+      s_tail[w] = tl_n;
+      tl_n += r;
     }
+    s_tail_base = tl_n ? atomicAdd(M.ctr + C_LIST, tl_n) : 0u;
+    s_seg_base = segs ? atomicAdd(M.ctr + C_SEGS, segs) : 0u;
     unsigned long long* st = reinterpret_cast<unsigned long long*>(M.ctr + C_STATS);
     if (pts) atomicAdd(st + S_POINTS, static_cast<unsigned long long>(pts));
     if (tl) atomicAdd(st + S_RAY_LEN, tl);
     s_base = tot ? atomicAdd(M.ctr + C_CAST, tot) : 0u;
   }
   __syncthreads();
+  uint32_t s_k = 0;
   if (add) {
     const uint32_t k = s_base + s_cnt[wid] + __popc(am & ((1u << lane) - 1));
     if (k < cast_cap)
       cast[k] = e;
     else
       set_err(M, ERR_SCRATCH);
+    s_k = k;
+    if ((tails >> lane) & 1u)
+      Q.tails[s_tail_base + s_tail[wid] + __popc(tails & ((1u << lane) - 1u))] = k;
+  }
+  // the warp's segments, number by number: neighbouring rays' segments lie side by side
+  uint32_t at = s_seg_base + s_seg[wid];
+  for (uint32_t j = 0;; ++j) {
+    const unsigned has = __ballot_sync(0xffffffffu, nseg > j);
+    if (!has) break;
+    if (nseg > j) Q.segs[at + __popc(has & ((1u << lane) - 1u))] = (s_k << 8) | j;
+    at += __popc(has);
   }
 }
 
@@ -238,69 +281,81 @@ __global__ void __launch_bounds__(U == 2 ? 256 : 1024, U == 2 ? 3 : 1) k_rays(co
   }
 }
 
-// Mark phase: block tasks of consecutive rays of the list (taken from the
-// counter *task, zero at launch), marked by mark_rays_block. Also clears
-// tab[0, tab_n), the scan's endpoint dedup table, for the next scan.
-__global__ void __launch_bounds__(1024) k_mark(const __grid_constant__ DMap M, RayCube Q,
-                                               const int4* __restrict__ cast, uint32_t cast_cap,
-                                               int ox, int oy, int oz,
-                                               uint4* __restrict__ tab, uint32_t tab_n,
-                                               uint32_t* task) {
-  __shared__ uint32_t sm[kMarkSmemWords];
-  __shared__ MarkRays<1024> rays;
-  __shared__ uint32_t s_task;
+// Mark phase (mark_scan). Also clears tab[0, tab_n), the scan's endpoint dedup
+// table, for the next scan.
+__global__ void __launch_bounds__(kMarkThreads, kMarkBlocksPerSM) k_mark(
+    const __grid_constant__ DMap M, const __grid_constant__ ScanCube Q,
+    const int4* __restrict__ cast, uint32_t cast_cap, int ox, int oy, int oz,
+    uint4* __restrict__ tab, uint32_t tab_n) {
+  __shared__ MarkShared S;
   for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < tab_n; t += gridDim.x * blockDim.x)
     tab[t] = make_uint4(kNone, kNone, kNone, kNone);
-  for (int t = threadIdx.x; t < kMarkSmemWords; t += blockDim.x) sm[t] = 0u;
   const uint32_t n_cast = min(ld_volatile(M.ctr + C_CAST), cast_cap);
-  // one task per block (a task ends with the block's shared-memory flush)
-  const uint32_t chunk = max(1u, (n_cast + gridDim.x - 1) / gridDim.x);
-  const uint32_t n_tasks = (n_cast + chunk - 1) / chunk;
+  const uint32_t n_segs = ld_volatile(M.ctr + C_SEGS);
   uint32_t visited = 0;
-  for (;;) {
-    __syncthreads();
-    if (threadIdx.x == 0) s_task = atomicAdd(task, 1u);
-    __syncthreads();
-    const uint32_t t = s_task;
-    if (t >= n_tasks) break;
-    const uint32_t r0 = t * chunk;
-    mark_rays_block<kMarkNB, 1024>(M, Q, cast, r0, min(n_cast, r0 + chunk), ox, oy, oz, sm,
-                                   rays, visited);
-  }
+  mark_scan(M, Q, cast, n_cast, n_segs, blockIdx.x, gridDim.x, ox, oy, oz, S, visited);
   visited = __reduce_add_sync(0xffffffffu, visited);
   if ((threadIdx.x & 31) == 0 && visited)
     atomicAdd(reinterpret_cast<unsigned long long*>(M.ctr + C_STATS) + S_VISITED,
               static_cast<unsigned long long>(visited));
 }
 
-// List phase: the marked blocks onto the scan's list (one warp per 32 words
-// of the touched bitmap).
-__global__ void __launch_bounds__(256) k_list_touched(const __grid_constant__ DMap M, RayCube Q) {
-  const uint32_t chunks = (cube_touched_words(Q) + 31u) / 32u;
-  const uint32_t wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t c = wid; c < chunks; c += nw) list_touched(M, Q, c);
-}
-
-
-// Apply phase: a group of kApplyGroup lanes per listed leaf block; D: the
-// map's leaf directory (D.words == nullptr: none).
-__global__ void __launch_bounds__(256) k_apply_rays(const __grid_constant__ DMap M, RayCube Q, int32_t u, int32_t miss,
-                                                    int32_t cmin, LeafDir D) {
-  const uint32_t n = min(ld_volatile(Q.count), Q.cap);
-  const unsigned lane = threadIdx.x & 31;
-  const unsigned sl = lane & (kApplyGroup - 1), gbase = lane & ~unsigned(kApplyGroup - 1);
-  const unsigned gmask = ((1u << kApplyGroup) - 1u) << gbase;
-  const uint32_t gid = (blockIdx.x * blockDim.x + threadIdx.x) / kApplyGroup;
-  const uint32_t ng = (gridDim.x * blockDim.x) / kApplyGroup;
+// Apply phase (apply_scan).
+__global__ void __launch_bounds__(256, 6) k_apply_rays(const __grid_constant__ DMap M,
+                                                    const __grid_constant__ ScanCube Q, int32_t u,
+                                                    int32_t miss, int32_t cmin) {
+  __shared__ uint32_t pre[kRootFlagWords], sums[8];
+  const uint32_t n_roots = apply_roots(Q, pre, sums);
+  const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   uint32_t updated = 0;
-  for (uint32_t i = gid; i < n; i += ng)
-    apply_block(M, Q, Q.list[i], u, miss, cmin, sl, gbase, gmask, updated,
-                D.words ? &D : nullptr);
+  apply_scan(M, Q, n_roots, pre, gw, (gridDim.x * blockDim.x) >> 5, u, miss, cmin, updated);
   updated = __reduce_add_sync(0xffffffffu, updated);
-  if (lane == 0 && updated)
+  if ((threadIdx.x & 31) == 0 && updated)
     atomicAdd(reinterpret_cast<unsigned long long*>(M.ctr + C_STATS) + S_UPDATED,
               static_cast<unsigned long long>(updated));
+}
+
+// The parts of rays that the cube does not hold (cells k >= kin; all cells of a
+// ray of kMarkMaxRay cells or more), walked on the tree. A warp takes a piece of a
+// ray, 1 / kTailPieces of it and at least two steps of 32 cells: a walk is a
+// chain of dependent loads, about 4 us a step, and the rays that go far are few
+// (29 k points at 0.05 m with returns to 100 m: 16 us; with eight rays per warp and
+// pieces of 256 cells 125 us; the whole scan walked by k_rays 330 us, against 17
+// for k_mark, 25 for k_apply_rays and this). Without a list of them (rays queued
+// by addHitPoint/addMissPoint) all rays are looked at.
+constexpr uint32_t kTailPieces = 32;
+__global__ void __launch_bounds__(256) k_tail(const __grid_constant__ DMap M,
+                                              const __grid_constant__ ScanCube Q,
+                                              const int4* __restrict__ cast, uint32_t cast_cap,
+                                              int ox, int oy, int oz, int32_t u, int32_t miss,
+                                              int32_t cmin) {
+  const uint32_t n = Q.tails ? ld_volatile(M.ctr + C_LIST) : min(ld_volatile(M.ctr + C_CAST), cast_cap);
+  const unsigned lane = threadIdx.x & 31;
+  const uint64_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint64_t nw = (gridDim.x * blockDim.x) >> 5;
+  uint32_t visited = 0, updated = 0;
+  for (uint64_t t = gw; t < uint64_t(n) * kTailPieces; t += nw) {
+    const uint32_t i = uint32_t(t / kTailPieces), j = uint32_t(t % kTailPieces);
+    const int4 e = cast[Q.tails ? Q.tails[i] : i];
+    const uint32_t m = chebyshev(ox, oy, oz, e.x, e.y, e.z);
+    if (m <= Q.kin) continue;
+    if (m >= kMaxRayCells) {
+      if (lane == 0) set_err(M, ERR_RAY_TOO_LONG);
+      continue;
+    }
+    const uint32_t from = m < kMarkMaxRay ? Q.kin : 0u;
+    const uint32_t piece = max(64u, (((m - from) / kTailPieces + 32u) & ~31u));
+    if (from + j * piece < m)
+      walk_ray<32>(M, e, ox, oy, oz, u, miss, cmin, lane, 0u, 0xffffffffu, visited, updated,
+                   nullptr, from + j * piece, from + (j + 1) * piece);
+  }
+  visited = __reduce_add_sync(0xffffffffu, visited);
+  updated = __reduce_add_sync(0xffffffffu, updated);
+  if (lane == 0 && visited) {
+    unsigned long long* st = reinterpret_cast<unsigned long long*>(M.ctr + C_STATS);
+    atomicAdd(st + S_VISITED, static_cast<unsigned long long>(visited));
+    atomicAdd(st + S_UPDATED, static_cast<unsigned long long>(updated));
+  }
 }
 
 // isOccupied / isUnknown / isFree (probabilistic_map.cpp:56-75).
@@ -395,7 +450,8 @@ int reset_scan_stats(MapCore* m) {
 // Endpoint phase for n staged points (k_endpoints or k_endpoints_kind), then
 // the winners that join the ray list, then the endpoint updates.
 template <class Launch>
-int endpoint_phase(bxg_pmap_s* pm, uint32_t n, int ox, int oy, int oz, Launch&& launch_ep) {
+int endpoint_phase(bxg_pmap_s* pm, uint32_t n, int ox, int oy, int oz, const ScanCube& cube,
+                   Launch&& launch_ep) {
   MapCore* m = &pm->core;
   const uint32_t tcap = next_pow2(uint64_t(n) * 2);
   BXG_CUDA(m, m->s_ep.ensure(size_t(n) * 16));
@@ -414,10 +470,12 @@ int endpoint_phase(bxg_pmap_s* pm, uint32_t n, int ox, int oy, int oz, Launch&& 
   record(pm, 1);
   k_winners<<<blocks, 256, 0, m->stream>>>(m->dm, m->s_ep.as<int4>(), n, m->s_dedup.as<uint4>(),
                                            tcap - 1, ox, oy, oz, pm->update_count, opts_of(pm),
-                                           m->s_cast.as<int4>(), uint32_t(m->s_cast.cap / 16));
+                                           m->s_cast.as<int4>(), uint32_t(m->s_cast.cap / 16),
+                                           cube);
   BXG_LAUNCHED(m);
   record(pm, 2);
   pm->cast_ub = need;
+  pm->has_segs = cube.bits != nullptr;
   return BXG_OK;
 }
 
@@ -495,6 +553,57 @@ int leaf_dir_for_scan(bxg_pmap_s* pm, int ox, int oy, int oz, LeafDir* D, size_t
 }  // namespace bxg
 
 namespace bxg {
+int scan_cube(bxg_pmap_s* pm, int ox, int oy, int oz, double reach, uint64_t rays, ScanCube* Q,
+              bool* ok) {
+  MapCore* m = &pm->core;
+  *ok = false;
+  *Q = ScanCube{};
+  if (m->dm.lb != 3 || m->dm.ib != 2 || m->dm.esz != 4 ||
+      (m->flags & (BXG_FLAG_KEEP_NONFINITE | BXG_FLAG_RAYS_SINGLE_PASS)))
+    return BXG_OK;
+  // Ray ends lie within ceil(reach / res) + 2 cells of the origin cell (the
+  // floor of the origin and of the end each move a cell by less than one).
+  const double cells = std::ceil(reach * m->inv_res) + 2.0;
+  int h = kOpenCubeHalf;
+  if (reach > 0 && cells <= 32.0 * kMaxCubeHalf)
+    h = std::max(1, (int(cells) + 31) / 32);
+  else
+    Q->open = 1;
+  Q->SR = uint32_t(2 * h + 1);
+  Q->S = 4 * Q->SR;
+  // cells k <= 32 h of a ray lie within h roots of the origin's
+  Q->kin = uint32_t(32 * h + 1);
+  const size_t blocks = size_t(Q->S) * Q->S * Q->S;
+  if (blocks > pm->cube_blocks) {
+    BXG_CUDA(m, pm->cube_bits.ensure(blocks * 64));
+    BXG_CUDA(m, cudaMemsetAsync(pm->cube_bits.p, 0, pm->cube_bits.cap, m->stream));
+    // the batched tick uses the buffers from another stream
+    BXG_CUDA(m, cudaStreamSynchronize(m->stream));
+    pm->cube_blocks = blocks;
+  }
+  if (!pm->cube_roots.p) {
+    BXG_CUDA(m, pm->cube_roots.ensure(kRootFlagWords * 4));
+    BXG_CUDA(m, cudaMemsetAsync(pm->cube_roots.p, 0, pm->cube_roots.cap, m->stream));
+  }
+  // a segment is a ray's position (24 bits) and a number (8 bits)
+  const uint64_t segs = rays * ((Q->kin - kNearCells + kSegCells - 1) / kSegCells);
+  if (rays && rays <= (1u << 24) && segs <= (1u << 28)) {
+    BXG_CUDA(m, pm->ray_segs.ensure(segs * 4));
+    Q->segs = pm->ray_segs.as<uint32_t>();
+  }
+  if (rays && Q->open) {
+    BXG_CUDA(m, pm->ray_tails.ensure(rays * 4));
+    Q->tails = pm->ray_tails.as<uint32_t>();
+  }
+  Q->bits = pm->cube_bits.as<uint32_t>();
+  Q->roots = pm->cube_roots.as<uint32_t>();
+  Q->x0 = ((ox >> 5) - h) * 32;
+  Q->y0 = ((oy >> 5) - h) * 32;
+  Q->z0 = ((oz >> 5) - h) * 32;
+  *ok = true;
+  return BXG_OK;
+}
+
 // Largest cube side (leaves): 200^3 blocks of 64 B = 512 MB of bits. Scans
 // whose cube would be larger (very fine resolutions with long ranges) walk
 // their rays with k_rays instead.
@@ -518,7 +627,8 @@ int cube_for_scan(bxg_pmap_s* pm, int ox, int oy, int oz, double reach, RayCube*
   if (S > kMaxCubeSide) return BXG_OK;
   const size_t blocks = size_t(S) * S * S;
   const uint32_t tmask = cube_touched_mask(S);
-  if (blocks > pm->cube_blocks) {
+  if (blocks > pm->cube_blocks || !pm->cube_touch.p ||
+      pm->cube_list.cap < blocks * 4 || pm->cube_touch.cap < (size_t(tmask) + 1) / 8) {
     BXG_CUDA(m, pm->cube_bits.ensure(blocks * 64));
     BXG_CUDA(m, pm->cube_touch.ensure((size_t(tmask) + 1) / 8));
     BXG_CUDA(m, pm->cube_list.ensure(blocks * 4));
@@ -526,7 +636,7 @@ int cube_for_scan(bxg_pmap_s* pm, int ox, int oy, int oz, double reach, RayCube*
     BXG_CUDA(m, cudaMemsetAsync(pm->cube_touch.p, 0, pm->cube_touch.cap, m->stream));
     // the batched tick uses the buffers from another stream
     BXG_CUDA(m, cudaStreamSynchronize(m->stream));
-    pm->cube_blocks = blocks;
+    pm->cube_blocks = std::max(pm->cube_blocks, blocks);
   }
   Q->bits = pm->cube_bits.as<uint32_t>();
   Q->touched = pm->cube_touch.as<uint32_t>();
@@ -567,38 +677,35 @@ int launch_rays(bxg_pmap_s* pm, int ox, int oy, int oz) {
   if (!pm->cast_ub) return BXG_OK;
   {
     // two-phase form: mark the rays' cells, then apply per leaf
-    RayCube Q{};
+    ScanCube Q;
     bool ok = false;
-    int st = cube_for_scan(pm, ox, oy, oz, pm->dir_reach, &Q, &ok);
+    int st = scan_cube(pm, ox, oy, oz, pm->dir_reach, pm->has_segs ? pm->cast_ub : 0, &Q, &ok);
     if (st) return st;
     if (ok) {
       const Opts o = opts_of(pm);
       const uint32_t ccap = uint32_t(m->s_cast.cap / 16);
       const uint32_t tab_n = m->dedup_used;
-      BXG_CUDA(m, cudaMemsetAsync(m->ctr.as<uint32_t>() + C_LIST, 0, 8, m->stream));
-      const unsigned mblocks =
-          unsigned(std::min<uint64_t>(m->sm_count, std::max<uint64_t>(1, pm->cast_ub / 64)));
-      k_mark<<<mblocks, 1024, 0, m->stream>>>(m->dm, Q, m->s_cast.as<int4>(), ccap, ox, oy, oz,
-                                             m->s_dedup.as<uint4>(), tab_n,
-                                             m->ctr.as<uint32_t>() + C_TASK);
+      // one resident wave, and no more blocks than have a ray or segment per thread
+      const uint64_t pieces = pm->cast_ub * (1 + (Q.kin - 1) / kSegCells);
+      const unsigned mblocks = unsigned(
+          std::min<uint64_t>(uint64_t(m->sm_count) * kMarkBlocksPerSM,
+                             (pieces + kMarkThreads - 1) / kMarkThreads));
+      k_mark<<<mblocks, kMarkThreads, 0, m->stream>>>(m->dm, Q, m->s_cast.as<int4>(), ccap, ox,
+                                                      oy, oz, m->s_dedup.as<uint4>(), tab_n);
       BXG_LAUNCHED(m);
-      const uint64_t chunks = (cube_touched_words(Q) + 31u) / 32u;
-      const unsigned lblocks =
-          unsigned(std::min<uint64_t>(uint64_t(m->sm_count) * 8, (chunks + 7) / 8));
-      k_list_touched<<<std::max(lblocks, 1u), 256, 0, m->stream>>>(m->dm, Q);
+      // the marked roots are at most those of the cube, or of the rays' pieces
+      const uint64_t rows = 16 * std::min<uint64_t>(uint64_t(Q.SR) * Q.SR * Q.SR, 8 * pieces);
+      const unsigned ablocks =
+          unsigned(std::min<uint64_t>(uint64_t(m->sm_count) * 12, (rows + 7) / 8));
+      k_apply_rays<<<ablocks, 256, 0, m->stream>>>(m->dm, Q, pm->update_count, o.miss, o.cmin);
       BXG_LAUNCHED(m);
-      // 256 / kApplyGroup groups per block; the list holds at most
-      // min(cube, 64 x rays) blocks
-      const uint64_t groups = std::min<uint64_t>(Q.cap, pm->cast_ub * 64);
-      const uint64_t per_block = 256 / kApplyGroup;
-      const unsigned ablocks = unsigned(std::min<uint64_t>(
-          uint64_t(m->sm_count) * 8, std::max<uint64_t>(1, (groups + per_block - 1) / per_block)));
-      LeafDir dir{};
-      st = leaf_dir_for_scan(pm, ox, oy, oz, &dir, size_t(1) << 24, m->stream);
-      if (st) return st;
-      k_apply_rays<<<ablocks, 256, 0, m->stream>>>(m->dm, Q, pm->update_count, o.miss, o.cmin,
-                                                   dir);
-      BXG_LAUNCHED(m);
+      if (Q.open) {
+        const unsigned tblocks = unsigned(std::min<uint64_t>(
+            uint64_t(m->sm_count) * 8, (pm->cast_ub * kTailPieces + 7) / 8));
+        k_tail<<<tblocks, 256, 0, m->stream>>>(m->dm, Q, m->s_cast.as<int4>(), ccap, ox, oy, oz,
+                                               pm->update_count, o.miss, o.cmin);
+        BXG_LAUNCHED(m);
+      }
       m->dedup_clean = std::max(m->dedup_clean, tab_n);
       m->dedup_used = 0;
       return BXG_OK;
@@ -767,21 +874,29 @@ int insert_impl(bxg_pmap m_, const PT* xyz, size_t stride, size_t n, const PT* o
     // rays of this scan end within max_range of the origin (hits are closer);
     // rays queued by earlier add batches may not: no directory then
     pm->dir_reach = pm->cast_ub == 0 ? max_range : 0.0;
-    const int zero = ZERO_STATS | (pm->cast_ub == 0 ? ZERO_CAST : 0);
+    // the winners cut the rays of a scan that starts its list into segments
+    ScanCube cube{};
+    if (pm->cast_ub == 0) {
+      bool ok = false;
+      st = scan_cube(pm, o[0], o[1], o[2], max_range, n, &cube, &ok);
+      if (st) return st;
+    }
+    const uint32_t root_words = cube.roots ? cube_root_words(cube) : 0;
+    const int zero = ZERO_STATS | ZERO_RAYS | (pm->cast_ub == 0 ? ZERO_CAST : 0);
     EpFast fast = make_ep_fast(fx, fy, fz, max_range, m->inv_res);
     if (sizeof(PT) != 4) fast.on = 0;
-    st = endpoint_phase(pm, uint32_t(n), o[0], o[1], o[2],
+    st = endpoint_phase(pm, uint32_t(n), o[0], o[1], o[2], cube,
                         [&](unsigned blocks, int4* ep, uint4* tab, uint32_t tmask) {
                           if (xf)
                             k_endpoints_sensor<<<blocks, 256, 0, m->stream>>>(
                                 m->dm, static_cast<const uint8_t*>(dpts), stride, uint32_t(n),
                                 *xf, fx, fy, fz, max_range, mr2, m->inv_res, ep, tab, tmask, zero,
-                                fast);
+                                fast, cube.roots, root_words);
                           else
                             k_endpoints<PT><<<blocks, 256, 0, m->stream>>>(
                                 m->dm, static_cast<const uint8_t*>(dpts), stride, uint32_t(n), fx,
                                 fy, fz, max_range, mr2, m->inv_res, keep, ep, tab, tmask, zero,
-                                fast);
+                                fast, cube.roots, root_words);
                         });
     if (st) return st;
   }
@@ -823,7 +938,7 @@ int add_points(bxg_pmap m_, const double* xyz, size_t n, int kind,
     st = stage_in(m, m->s_in2, kinds, n, &dkinds);
     if (st) return st;
   }
-  st = endpoint_phase(pm, uint32_t(n), 0, 0, 0,
+  st = endpoint_phase(pm, uint32_t(n), 0, 0, 0, ScanCube{},
                       [&](unsigned blocks, int4* ep, uint4* tab, uint32_t tmask) {
                         k_endpoints_kind<<<blocks, 256, 0, m->stream>>>(
                             m->dm, static_cast<const double*>(dpts), uint32_t(n), kind,

@@ -255,7 +255,7 @@ __device__ __forceinline__ bool winner_apply(const DMap& M, int4 e, int32_t u, c
 // walk_ray_op is the walk itself; per step every lane calls
 // op(act, leaf, ci, k): act = the lane has a cell (k < m), leaf = its leaf
 // slot (kNone if the pool ran out), ci = its index in the leaf, k = its
-// position on the ray.
+// position on the ray. k0, k1: only the cells k0 <= k < k1 of the ray.
 // Leaf directory: a dense cube of `side`^3 words over the leaves around the
 // scan's origin, covering every leaf within max_range (x0/y0/z0: leaf
 // coordinate of its corner). A word holds (epoch << 28) | leaf slot; a word of
@@ -276,7 +276,8 @@ struct LeafDir {
 template <int W, bool DIR, class Op>
 __device__ __forceinline__ void walk_ray_op(const DMap& M, int4 e, int ox, int oy, int oz,
                                             unsigned sl, unsigned gbase, unsigned gmask,
-                                            Op&& op, const LeafDir* D) {
+                                            Op&& op, const LeafDir* D, uint32_t k0 = 0,
+                                            uint32_t k1 = kNone) {
   const int dx = e.x - ox, dy = e.y - oy, dz = e.z - oz;
   const uint32_t ax = static_cast<uint32_t>(abs(dx)), ay = static_cast<uint32_t>(abs(dy)),
                  az = static_cast<uint32_t>(abs(dz));
@@ -295,11 +296,17 @@ __device__ __forceinline__ void walk_ray_op(const DMap& M, int4 e, int ox, int o
   axis_init(X, ax, m, two_m, rtm, sl, W);
   axis_init(Y, ay, m, two_m, rtm, sl, W);
   axis_init(Z, az, m, two_m, rtm, sl, W);
+  if (k0) {  // a piece of the ray: its own start, in 64 bits (k0 d may pass 2^31)
+    axis_start64(X, ax, m, k0 + sl);
+    axis_start64(Y, ay, m, k0 + sl);
+    axis_start64(Z, az, m, k0 + sl);
+  }
+  const uint32_t end = min(m, k1);
   uint32_t pkey = kNone;  // packed leaf index of the previous step's last lane
   uint32_t pleaf = kNone;
 
-  for (uint32_t base = 0; base < m; base += W) {
-    const bool act = base + sl < m;
+  for (uint32_t base = k0; base < end; base += W) {
+    const bool act = base + sl < end;
     const int cx = ox + sx * static_cast<int>(X.n);
     const int cy = oy + sy * static_cast<int>(Y.n);
     const int cz = oz + sz * static_cast<int>(Z.n);
@@ -342,7 +349,7 @@ __device__ __forceinline__ void walk_ray_op(const DMap& M, int4 e, int ox, int o
     const uint32_t got = __shfl_sync(gmask, leaf, below ? 31 - __clz(below) : 0, W);
     leaf = below ? got : pleaf;
     op(act, leaf, leaf_index(M, cx, cy, cz), base + sl);
-    const uint32_t rem = m - base;
+    const uint32_t rem = end - base;
     const int last = static_cast<int>(rem < W ? rem : W) - 1;
     pkey = __shfl_sync(gmask, key, last, W);
     pleaf = __shfl_sync(gmask, leaf, last, W);
@@ -357,7 +364,8 @@ template <int W, bool DIR = false>
 __device__ __forceinline__ void walk_ray(const DMap& M, int4 e, int ox, int oy, int oz,
                                          int32_t u, int32_t miss, int32_t cmin, unsigned sl,
                                          unsigned gbase, unsigned gmask, uint32_t& visited,
-                                         uint32_t& updated, const LeafDir* D = nullptr) {
+                                         uint32_t& updated, const LeafDir* D = nullptr,
+                                         uint32_t k0 = 0, uint32_t k1 = kNone) {
   int32_t* const cells = reinterpret_cast<int32_t*>(M.ldata);
   walk_ray_op<W, DIR>(M, e, ox, oy, oz, sl, gbase, gmask,
                  [&](bool act, uint32_t leaf, uint32_t ci, uint32_t) {
@@ -372,7 +380,7 @@ __device__ __forceinline__ void walk_ray(const DMap& M, int4 e, int ox, int oy, 
                      visited++;
                    }
                  },
-                 D);
+                 D, k0, k1);
 }
 
 // Leaf slot of a head cell: the inline hash probe, else the bounded-wait
