@@ -1,29 +1,32 @@
 // Batched form: one insertPointCloud scan for each of many independent maps
-// per tick, in ONE persistent cooperative launch captured in a CUDA graph.
+// per tick, as a few launches captured in a CUDA graph.
 //
 // The per-map scan (bxg_pmap.cu) is four small launches with a host sync; a
 // 10k-point scan cannot fill 152 SMs, so many small maps spend their time in
 // launch and sync latency. Here every phase covers all scans of the tick:
 //
-//   phase 0  clear the dedup tables and per-scan counters
-//   phase 1  endpoints of every point of every scan (compute_endpoint),
-//            lowest index per endpoint cell in the scan's own table
-//   phase 2  winners apply their hit/miss and join their scan's ray list
-//   phase 3  prefix sum of the ray-list lengths (one global ray index space)
-//   phase 4  the ray phase of all scans. Two-phase form (every map has a
-//            cube bitmap, bxg_mark.cuh): 4a blocks take tasks of consecutive
-//            rays of one scan and mark their cells in that map's bitmap; 4b
-//            warps list the marked leaf blocks of every map; 4c groups of 8
-//            lanes apply each map's listed blocks. Single-pass
-//            form otherwise: groups of W lanes walk rays of all scans
-//            (walk_ray), each on its own map's pools. Statistics per scan.
-//   phase 5  each map's counters are copied to one read-back block
+//   k_tick_begin      clears the dedup tables, counters and root bits
+//   k_tick_endpoints  endpoints of every point of every scan, lowest index per
+//                     endpoint cell in the scan's own table
+//   k_tick_winners    winners apply their hit/miss, join their scan's ray list and
+//                     list their segments
+//   k_tick_mark       the ray cells of all scans into their maps' bitmaps
+//   k_tick_roots      the marked roots of all maps on one list
+//   k_tick_apply      each marked leaf's cells (bxg_mark.cuh for these phases)
+//   k_tick_tail       only with scans whose rays may leave their cube
+//   k_tick_end        each map's counters into one read-back block
 //
-// separated by grid barriers (bounded waits: a barrier that times out sets an
-// error word and the kernel returns). Each map keeps its own pools; the tick
-// touches no state shared between maps except the read-only descriptors. The
-// arithmetic is exactly that of the per-map path (bxg_scan.cuh), so the maps
-// are bit-identical to inserting the scans one by one.
+// The grids are one or two resident waves, whatever the tick holds, so that one
+// captured graph serves ticks of any sizes. Separate launches instead of phases of one
+// persistent kernel let each have its own registers, shared memory and occupancy.
+// When a map keeps non-finite points or asks for the single-pass ray phase, the tick
+// runs as that persistent cooperative kernel (k_tick): the same phases separated by grid
+// barriers, and rays walked on the tree by groups of W lanes.
+//
+// Each map keeps its own pools and counters; the tick touches no state shared
+// between maps except the read-only descriptors. The arithmetic is exactly that
+// of the per-map path (bxg_scan.cuh, bxg_mark.cuh), so the maps are
+// bit-identical to inserting the scans one by one.
 #include <algorithm>
 #include <cstring>
 #include <vector>
@@ -46,11 +49,8 @@ constexpr size_t kOffCnt = kOffStats + kMaxTickScans * 32;       // [128] u32
 constexpr size_t kOffCtr = kOffCnt + kMaxTickScans * 4;          // [128][C_WORDS] u32
 constexpr size_t kBackBytes = kOffCtr + kMaxTickScans * C_WORDS * 4;
 constexpr size_t kOffPrefix = kBackBytes;                        // [129] u32
-constexpr size_t kOffTaskPrefix = kOffPrefix + (kMaxTickScans + 1) * 4;  // [129] u32
-constexpr size_t kOffChunk = kOffTaskPrefix + (kMaxTickScans + 1) * 4;   // u32
-constexpr size_t kMetaBytes = kOffChunk + 16;
-// The tick's neighbourhood of shared-memory leaves around each scan's origin.
-constexpr int kTickMarkNB = 2;
+constexpr size_t kOffRoots = kOffPrefix + (kMaxTickScans + 1) * 4;  // u32
+constexpr size_t kMetaBytes = kOffRoots + 16;
 
 struct TickScan {
   DMap M;
@@ -63,9 +63,9 @@ struct TickScan {
   uint32_t n;                    // points
   uint32_t tmask;                // dedup table size - 1
   int32_t keep_nonfinite;
-  uint32_t chunk0;  // first chunk (32 touched words) of this scan's cube in the tick's list phase
-  RayCube Q;  // the map's cube bitmap (two-phase ray update)
-  LeafDir D;  // the map's kept leaf directory (D.words == nullptr: none)
+  uint32_t chunk0;      // first of the scan's chunks of 256 points
+  unsigned long long root0;  // first word of the scan's root bits, over all scans
+  ScanCube Q;           // the map's cube (two-phase ray update)
 };
 
 static_assert(sizeof(TickScan) % 8 == 0, "TickScan is copied to shared memory in 8-byte words");
@@ -80,13 +80,14 @@ struct TickArgs {
   uint32_t* ray_prefix;       // [n_scans + 1]
   uint32_t* bar;              // barrier: arrivals, generation
   uint32_t* err;              // barrier timeout
-  uint32_t* ray_next;         // next ray (or mark task) taken in phase 4 (zeroed per tick)
-  uint32_t* task_prefix;      // [n_scans + 1] first mark task of each scan
-  uint32_t* chunk;            // rays per mark task
+  uint32_t* ray_next;         // next ray (or mark task) taken (zeroed per tick)
+  uint32_t* roots;            // marked roots: scan << 17 | root
+  uint32_t* n_roots;
   uint32_t* ctr_out;          // [n_scans][C_WORDS]
   unsigned long long* times;  // [8] global-timer stamps at each phase boundary
   uint32_t n_scans;
-  uint32_t n_chunks;  // chunks of 32 touched words over all scans' cubes
+  uint32_t n_chunks;  // chunks of 256 points over all scans
+  unsigned long long root_words;  // words of root bits over all scans
   unsigned long long total_points;
   unsigned long long total_tab;
 };
@@ -151,17 +152,35 @@ __device__ __forceinline__ uint32_t scan_of_ray(const uint32_t* prefix, uint32_t
   return lo;
 }
 
-__device__ __forceinline__ uint32_t scan_of_task(const uint32_t* prefix, uint32_t n, uint32_t t) {
-  uint32_t lo = 0, hi = n;  // last scan with prefix <= t (scans without tasks are skipped)
-  while (hi - lo > 1) {
-    const uint32_t mid = (lo + hi) >> 1;
-    if (ld_volatile(prefix + mid) <= t) lo = mid; else hi = mid;
+// ---------------------------------------------------------------------------
+// the launches of a tick in the two-phase form
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void tick_stamp(const TickArgs& A, int k) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) A.times[k] = global_ns();
+}
+
+__global__ void __launch_bounds__(256) k_tick_begin(const TickArgs* __restrict__ argp,
+                                                    const TickScan* __restrict__ sc) {
+  const TickArgs& A = *argp;
+  tick_stamp(A, 0);
+  const unsigned long long gtid = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
+  const unsigned long long gsize = gridDim.x * (unsigned long long)blockDim.x;
+  const uint4 kEmpty = make_uint4(kNone, kNone, kNone, kNone);
+  for (unsigned long long k = gtid; k < A.total_tab; k += gsize) A.tab[k] = kEmpty;
+  // a block per scan: its counters and root bits
+  for (uint32_t s = blockIdx.x; s < A.n_scans; s += gridDim.x) {
+    uint32_t* ctr = sc[s].M.ctr;
+    const uint32_t words = cube_root_words(sc[s].Q);
+    for (uint32_t t = threadIdx.x; t < words; t += blockDim.x) sc[s].Q.roots[t] = 0u;
+    if (threadIdx.x < S_COUNT)
+      reinterpret_cast<unsigned long long*>(ctr + C_STATS)[threadIdx.x] = 0ull;
+    if (threadIdx.x == 32) ctr[C_CAST] = ctr[C_SEGS] = ctr[C_TAILS] = 0u;
   }
-  return lo;
+  if (gtid == 0) *A.n_roots = 0u;
 }
 
 __device__ __forceinline__ uint32_t scan_of_chunk(const TickScan* sc, uint32_t n, uint32_t c) {
-  uint32_t lo = 0, hi = n;  // last scan with chunk0 <= c
+  uint32_t lo = 0, hi = n;  // last scan with chunk0 <= c (scans without points are skipped)
   while (hi - lo > 1) {
     const uint32_t mid = (lo + hi) >> 1;
     if (sc[mid].chunk0 <= c) lo = mid; else hi = mid;
@@ -169,19 +188,202 @@ __device__ __forceinline__ uint32_t scan_of_chunk(const TickScan* sc, uint32_t n
   return lo;
 }
 
-// MARK: phase 4 in the two-phase form (every scan has a cube). Dynamic shared
-// memory: the scan table (n_scans entries), then, with MARK, the mark
-// neighbourhood (mark_smem_words(kTickMarkNB) words).
-template <int W, int U, bool MARK>
+__global__ void __launch_bounds__(256) k_tick_endpoints(const TickArgs* __restrict__ argp,
+                                                        const TickScan* __restrict__ sc) {
+  const TickArgs& A = *argp;
+  tick_stamp(A, 1);
+  for (uint32_t c = blockIdx.x; c < A.n_chunks; c += gridDim.x) {
+    const TickScan& S = sc[scan_of_chunk(sc, A.n_scans, c)];
+    const uint32_t i = (c - S.chunk0) * 256u + threadIdx.x;
+    int4 e = make_int4(0, 0, 0, EP_SKIP);
+    if (i < S.n) {
+      const float* p = reinterpret_cast<const float*>(A.pts) + 3 * (S.pt_begin + i);
+      e = compute_endpoint<float>(p, S.fx, S.fy, S.fz, S.max_range, S.mr2, S.inv_res,
+                                  S.keep_nonfinite != 0, &S.fast);
+    }
+    endpoint_enter(S.M, e, i, A.tab + S.tab_begin, S.tmask);
+    if (i < S.n) A.ep[S.pt_begin + i] = e;
+  }
+}
+
+// 32 registers for eight blocks per SM: 0.33 ms for 8 M points of 64 maps (48 registers
+// and five blocks 0.48 ms: the chain of table, root, leaf and cell loads wants warps).
+__global__ void __launch_bounds__(256, 8) k_tick_winners(const TickArgs* __restrict__ argp,
+                                                      const TickScan* __restrict__ sc) {
+  __shared__ WinnersShared W;
+  const TickArgs& A = *argp;
+  tick_stamp(A, 2);
+  for (uint32_t c = blockIdx.x; c < A.n_chunks; c += gridDim.x) {
+    const TickScan& S = sc[scan_of_chunk(sc, A.n_scans, c)];
+    winners_block(S.M, A.ep + S.pt_begin, S.n, (c - S.chunk0) * 256u + threadIdx.x,
+                  A.tab + S.tab_begin, S.tmask, S.ox, S.oy, S.oz, S.u, S.o, A.cast + S.pt_begin,
+                  S.n, S.Q, W);
+    __syncthreads();
+  }
+}
+
+// Tasks are equal shares of the rays (near cells) and segments of all scans, about four
+// per block, taken as blocks become free; at least one piece per thread, so that a small
+// tick reaches every SM (8 maps of 2-20 k points: 31 us; with shares of 2048 pieces 112 us).
+// 64 maps, 674 M cells: 1.47 ms (2.69 ms as a phase of the persistent kernel, with
+// segments found by a prefix per 256 rays), bound by instruction issue.
+__global__ void __launch_bounds__(kMarkThreads, kMarkBlocksPerSM) k_tick_mark(
+    const TickArgs* __restrict__ argp, const TickScan* __restrict__ sc) {
+  __shared__ MarkShared S;
+  __shared__ unsigned long long pre[kMaxTickScans + 1];
+  __shared__ uint32_t s_task;
+  const TickArgs& A = *argp;
+  tick_stamp(A, 4);
+  const uint32_t ns = A.n_scans;
+  if (threadIdx.x < ns) {
+    const TickScan& T = sc[threadIdx.x];
+    pre[threadIdx.x + 1] = (unsigned long long)min(T.M.ctr[C_CAST], T.n) +
+                           (T.Q.segs ? T.M.ctr[C_SEGS] : 0u);
+  }
+  if (threadIdx.x == 0) pre[0] = 0ull;
+  __syncthreads();
+  if (threadIdx.x == 0)
+    for (uint32_t s = 0; s < ns; ++s) pre[s + 1] += pre[s];
+  __syncthreads();
+  const unsigned long long total = pre[ns];
+  const unsigned long long tasks = min(4ull * gridDim.x, total / kMarkThreads + 1ull);
+  for (;;) {
+    __syncthreads();
+    if (threadIdx.x == 0) s_task = atomicAdd(A.ray_next, 1u);
+    __syncthreads();
+    const unsigned long long t = s_task;
+    if (t >= tasks) break;
+    unsigned long long lo = total * t / tasks;
+    const unsigned long long end = total * (t + 1) / tasks;
+    uint32_t s = 0, hi = ns;  // last scan that starts at or before lo
+    while (hi - s > 1) {
+      const uint32_t mid = (s + hi) >> 1;
+      if (pre[mid] <= lo) s = mid; else hi = mid;
+    }
+    for (; lo < end; ++s) {
+      const unsigned long long stop = min(end, pre[s + 1]);
+      if (lo >= stop) continue;
+      const TickScan& T = sc[s];
+      const ScanCube Q = T.Q;  // in registers: the ORs keep the compiler from holding loads
+      const uint32_t n = min(T.M.ctr[C_CAST], T.n);
+      const uint32_t a = uint32_t(lo - pre[s]), b = uint32_t(stop - pre[s]);
+      uint32_t visited = 0;
+      mark_scan(T.M, Q, A.cast + T.pt_begin, min(a, n), min(b, n), max(a, n) - n, max(b, n) - n,
+                kMarkThreads, T.ox, T.oy, T.oz, S, visited);
+      visited = __reduce_add_sync(0xffffffffu, visited);
+      if ((threadIdx.x & 31) == 0 && visited)
+        atomicAdd(reinterpret_cast<unsigned long long*>(T.M.ctr + C_STATS) + S_VISITED,
+                  static_cast<unsigned long long>(visited));
+      lo = stop;
+    }
+  }
+}
+
+__global__ void __launch_bounds__(256) k_tick_roots(const TickArgs* __restrict__ argp,
+                                                    const TickScan* __restrict__ sc) {
+  const TickArgs& A = *argp;
+  tick_stamp(A, 6);
+  const unsigned lane = threadIdx.x & 31;
+  const unsigned long long gsize = gridDim.x * (unsigned long long)blockDim.x;
+  for (unsigned long long w0 = blockIdx.x * (unsigned long long)blockDim.x + (threadIdx.x & ~31u);
+       w0 < A.root_words; w0 += gsize) {
+    const unsigned long long w = w0 + lane;
+    uint32_t v = 0, s = 0, i = 0;
+    if (w < A.root_words) {
+      uint32_t hi = A.n_scans;  // last scan whose words start at or before w
+      while (hi - s > 1) {
+        const uint32_t mid = (s + hi) >> 1;
+        if (sc[mid].root0 <= w) s = mid; else hi = mid;
+      }
+      const ScanCube& Q = sc[s].Q;
+      i = uint32_t(w - sc[s].root0);
+      v = Q.roots[i];
+      const uint32_t bits = Q.SR * Q.SR * Q.SR;
+      if (32u * i + 32u > bits) v &= (1u << (bits & 31u)) - 1u;
+    }
+    const uint32_t cnt = __popc(v);
+    uint32_t incl = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t x = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= unsigned(o)) incl += x;
+    }
+    const uint32_t tot = __shfl_sync(0xffffffffu, incl, 31);
+    if (!tot) continue;
+    uint32_t base = 0;
+    if (lane == 0) base = atomicAdd(A.n_roots, tot);
+    uint32_t k = __shfl_sync(0xffffffffu, base, 0) + incl - cnt;
+    for (; v; v &= v - 1u) A.roots[k++] = (s << 17) | (32u * i + uint32_t(__ffs(v) - 1));
+  }
+}
+
+// 64 maps, 318 M updated cells: 1.28 ms (1.5 ms as a phase of the persistent kernel, eight
+// lanes per leaf), bound by the DRAM sectors of the cells; eight blocks per SM, and four
+// times as many blocks as that, to even out rows of very different work (one such wave: 1.32 ms).
+__global__ void __launch_bounds__(256, 8) k_tick_apply(const TickArgs* __restrict__ argp,
+                                                       const TickScan* __restrict__ sc) {
+  __shared__ ApplyShared W;
+  const TickArgs& A = *argp;
+  tick_stamp(A, 7);
+  const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
+  const uint32_t n = 16u * *A.n_roots;
+  uint32_t updated = 0, cur = kNone;
+  auto count = [&]() {
+    updated = __reduce_add_sync(0xffffffffu, updated);
+    if ((threadIdx.x & 31) == 0 && updated)
+      atomicAdd(reinterpret_cast<unsigned long long*>(sc[cur].M.ctr + C_STATS) + S_UPDATED,
+                static_cast<unsigned long long>(updated));
+    updated = 0;
+  };
+  for (uint32_t t = gw; t < n; t += nw) {
+    const uint32_t e = A.roots[t >> 4], s = e >> 17, i = e & 0x1FFFFu;
+    if (s != cur) {
+      if (cur != kNone) count();
+      cur = s;
+    }
+    const TickScan& T = sc[s];
+    const uint32_t SR = T.Q.SR;
+    const uint32_t rz = i / (SR * SR), ry = (i - rz * SR * SR) / SR, rx = i - (rz * SR + ry) * SR;
+    apply_row(T.M, T.Q, rx, 4u * ry + (t & 3u), 4u * rz + ((t >> 2) & 3u), T.u, T.o.miss, T.o.cmin,
+              W.rows[threadIdx.x >> 5], updated);
+  }
+  if (cur != kNone) count();
+}
+
+__global__ void __launch_bounds__(256) k_tick_tail(const TickArgs* __restrict__ argp,
+                                                   const TickScan* __restrict__ sc) {
+  const TickArgs& A = *argp;
+  const uint64_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint64_t nw = (gridDim.x * blockDim.x) >> 5;
+  for (uint32_t s = 0; s < A.n_scans; ++s) {
+    const TickScan& T = sc[s];
+    if (!T.Q.open) continue;
+    uint32_t visited = 0, updated = 0;
+    tail_rays(T.M, T.Q, A.cast + T.pt_begin, T.n, gw, nw, T.ox, T.oy, T.oz, T.u, T.o.miss,
+              T.o.cmin, visited, updated);
+    tail_count(T.M, visited, updated);
+  }
+}
+
+__global__ void __launch_bounds__(256) k_tick_end(const TickArgs* __restrict__ argp,
+                                                  const TickScan* __restrict__ sc) {
+  const TickArgs& A = *argp;
+  tick_stamp(A, 5);
+  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < A.n_scans * C_WORDS;
+       k += gridDim.x * blockDim.x)
+    A.ctr_out[k] = sc[k / C_WORDS].M.ctr[k % C_WORDS];
+}
+
+// The whole tick with the single-pass ray phase, as one persistent cooperative
+// launch. Dynamic shared memory: the scan table (n_scans entries).
+template <int W, int U>
 __global__ void __launch_bounds__(256, U == 2 ? 3 : 4) k_tick(const TickArgs* __restrict__ argp,
                                                  const TickScan* __restrict__ scans_g) {
   extern __shared__ unsigned long long smem_raw[];
   TickScan* sc = reinterpret_cast<TickScan*>(smem_raw);
-  __shared__ uint32_t s_task;
-  __shared__ uint32_t s_upd[kMaxTickScans];
   const TickArgs A = *argp;
   const uint32_t ns = A.n_scans;
-  uint32_t* smk = reinterpret_cast<uint32_t*>(smem_raw + ns * (sizeof(TickScan) / 8));
   {
     const uint32_t words = ns * (sizeof(TickScan) / 8);
     const unsigned long long* src = reinterpret_cast<const unsigned long long*>(scans_g);
@@ -202,7 +404,6 @@ __global__ void __launch_bounds__(256, U == 2 ? 3 : 4) k_tick(const TickArgs* __
   for (unsigned long long k = gtid; k < ns; k += gsize) {
     A.cast_cnt[k] = 0;
     for (int j = 0; j < 4; j++) A.stats[4 * k + j] = 0;
-    if (MARK) *sc[k].Q.count = 0u;  // the list phase appends from zero
   }
   if (!grid_barrier(A.bar, A.err)) return;
   stamp(1);
@@ -268,8 +469,7 @@ __global__ void __launch_bounds__(256, U == 2 ? 3 : 4) k_tick(const TickArgs* __
   if (!grid_barrier(A.bar, A.err)) return;
   stamp(3);
 
-  // phase 3: one index space over all ray lists (and, with MARK, over the
-  // mark tasks: about four per block, at least 64 rays each)
+  // phase 3: one index space over all ray lists
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     uint32_t acc = 0;
     for (uint32_t s = 0; s < ns; s++) {
@@ -277,79 +477,12 @@ __global__ void __launch_bounds__(256, U == 2 ? 3 : 4) k_tick(const TickArgs* __
       acc += min(ld_volatile(A.cast_cnt + s), sc[s].n);
     }
     A.ray_prefix[ns] = acc;
-    if (MARK) {
-      const uint32_t chunk = max(64u, (acc + 4u * gridDim.x - 1) / (4u * gridDim.x));
-      uint32_t tacc = 0;
-      for (uint32_t s = 0; s < ns; s++) {
-        A.task_prefix[s] = tacc;
-        tacc += (A.ray_prefix[s + 1] - A.ray_prefix[s] + chunk - 1) / chunk;
-      }
-      A.task_prefix[ns] = tacc;
-      *A.chunk = chunk;
-    }
   }
   if (!grid_barrier(A.bar, A.err)) return;
   stamp(4);
 
   // phase 4: rays of all scans
-  if (MARK) {
-    // 4a: mark
-    __shared__ MarkRays<256> s_rays;
-    for (int t = threadIdx.x; t < mark_smem_words(kTickMarkNB); t += blockDim.x) smk[t] = 0u;
-    const uint32_t n_tasks = ld_volatile(A.task_prefix + ns);
-    const uint32_t chunk = ld_volatile(A.chunk);
-    for (;;) {
-      __syncthreads();
-      if (threadIdx.x == 0) s_task = atomicAdd(A.ray_next, 1u);
-      __syncthreads();
-      const uint32_t t = s_task;
-      if (t >= n_tasks) break;
-      const uint32_t s = scan_of_task(A.task_prefix, ns, t);
-      const TickScan& S = sc[s];
-      const uint32_t rays = ld_volatile(A.ray_prefix + s + 1) - ld_volatile(A.ray_prefix + s);
-      const uint32_t r0 = (t - ld_volatile(A.task_prefix + s)) * chunk;
-      uint32_t visited = 0;
-      mark_rays_block<kTickMarkNB, 256>(S.M, S.Q, A.cast + S.pt_begin, r0, min(rays, r0 + chunk),
-                                        S.ox, S.oy, S.oz, smk, s_rays, visited);
-      visited = __reduce_add_sync(0xffffffffu, visited);
-      if (lane == 0 && visited)
-        atomicAdd(A.stats + 4 * s + 2, static_cast<unsigned long long>(visited));
-    }
-    if (!grid_barrier(A.bar, A.err)) return;
-    stamp(6);
-    // 4b: the marked blocks of every cube onto its list (a warp per 32
-    // touched words, all scans in one index space)
-    for (uint32_t c = static_cast<uint32_t>(gtid >> 5); c < A.n_chunks;
-         c += static_cast<uint32_t>(gsize >> 5)) {
-      const uint32_t s = scan_of_chunk(sc, ns, c);
-      list_touched(sc[s].M, sc[s].Q, c - sc[s].chunk0);
-    }
-    if (!grid_barrier(A.bar, A.err)) return;
-    stamp(7);
-    // 4c: apply, 8 lanes per listed leaf block; each scan's list is taken in
-    // a rotated order so that its first entries do not always go to the same
-    // groups
-    for (uint32_t k = threadIdx.x; k < ns; k += blockDim.x) s_upd[k] = 0u;
-    __syncthreads();
-    {
-      const unsigned sl = lane & (kApplyGroup - 1), gbase = lane & ~unsigned(kApplyGroup - 1);
-      const unsigned gmask = ((1u << kApplyGroup) - 1u) << gbase;
-      const uint32_t gid = static_cast<uint32_t>(gtid / kApplyGroup);
-      const uint32_t ng = static_cast<uint32_t>(gsize / kApplyGroup);
-      for (uint32_t s = 0; s < ns; ++s) {
-        const TickScan& S = sc[s];
-        const uint32_t n = min(ld_volatile(S.Q.count), S.Q.cap);
-        uint32_t upd = 0;
-        for (uint32_t i = (gid + s * 977u) % ng; i < n; i += ng)
-          apply_block(S.M, S.Q, S.Q.list[i], S.u, S.o.miss, S.o.cmin, sl, gbase, gmask, upd,
-                      S.D.words ? &S.D : nullptr);
-        if (upd) atomicAdd(s_upd + s, upd);
-      }
-    }
-    __syncthreads();
-    for (uint32_t k = threadIdx.x; k < ns; k += blockDim.x)
-      if (s_upd[k]) atomicAdd(A.stats + 4 * k + 3, static_cast<unsigned long long>(s_upd[k]));
-  } else {
+  {
     const unsigned sl = lane & (W - 1);
     const unsigned gbase = lane & ~(W - 1);
     const unsigned gmask = (W == 32) ? 0xffffffffu : (((1u << W) - 1u) << gbase);
@@ -417,12 +550,12 @@ struct bxg_batch_s {
   uint32_t rays_per_warp = 1;
   uint32_t ray_unroll = 1;
   int sm_count = 0;
-  int grid = 0;       // resident blocks of the single-pass tick
-  int grid_mark = 0;  // resident blocks of the two-phase tick
-  size_t grid_smem[2] = {0, 0};  // dynamic shared memory the two were sized for
+  int grid = 0;          // resident blocks of the single-pass tick
+  size_t grid_smem = 0;  // dynamic shared memory that was sized for
+  int grid_mark = 0;     // blocks of the two-phase tick's mark phase
   bool use_graph = true;
   // device buffers
-  DevBuf pts, ep, tab, cast, meta, params;
+  DevBuf pts, ep, tab, cast, segs, tails, roots, meta, params;
   // pinned host staging
   TickArgs* h_args = nullptr;
   TickScan* h_scans = nullptr;
@@ -432,7 +565,7 @@ struct bxg_batch_s {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   bool graph_ok = false;
-  uint64_t graph_key[7] = {0};
+  uint64_t graph_key[8] = {0};
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   float last_ms = 0;
   double phase_ms[6] = {0, 0, 0, 0, 0, 0};  // [5]: the mark part of the ray phase
@@ -472,10 +605,10 @@ uint32_t pow2_at_least(uint64_t v) {
   return p;
 }
 
-template <int W, int U, bool MARK>
+template <int W, int U>
 int occupancy_grid(bxg_batch b, size_t smem) {
   int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tick<W, U, MARK>, 256, smem) !=
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tick<W, U>, 256, smem) !=
       cudaSuccess) {
     cudaGetLastError();
     return 0;
@@ -483,16 +616,13 @@ int occupancy_grid(bxg_batch b, size_t smem) {
   return per_sm * b->sm_count;
 }
 
-// Dynamic shared memory of a tick of ns scans: the scan table, plus the mark
-// neighbourhood in the two-phase form.
-size_t tick_smem(bool mark, size_t ns) {
-  return ns * sizeof(TickScan) + (mark ? size_t(mark_smem_words(kTickMarkNB)) * 4 : 0);
-}
+// Dynamic shared memory of a single-pass tick of ns scans: the scan table.
+size_t tick_smem(size_t ns) { return ns * sizeof(TickScan); }
 
-template <int W, int U, bool MARK>
+template <int W, int U>
 cudaError_t launch_tick(bxg_batch b, size_t smem) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(MARK ? b->grid_mark : b->grid);
+  cfg.gridDim = dim3(b->grid);
   cfg.blockDim = dim3(256);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = b->stream;
@@ -503,27 +633,41 @@ cudaError_t launch_tick(bxg_batch b, size_t smem) {
   cfg.numAttrs = 1;
   const TickArgs* a = b->params.as<TickArgs>();
   const TickScan* s = reinterpret_cast<const TickScan*>(b->params.as<uint8_t>() + 256);
-  return cudaLaunchKernelEx(&cfg, k_tick<W, U, MARK>, a, s);
+  return cudaLaunchKernelEx(&cfg, k_tick<W, U>, a, s);
 }
 
-cudaError_t launch_for(bxg_batch b, size_t smem, bool mark) {
-  if (mark) return launch_tick<32, 1, true>(b, smem);
+cudaError_t launch_single_pass(bxg_batch b, size_t smem) {
   const bool u2 = b->ray_unroll == 2;
   switch (b->rays_per_warp) {
-    case 4: return u2 ? launch_tick<8, 2, false>(b, smem) : launch_tick<8, 1, false>(b, smem);
-    case 2: return u2 ? launch_tick<16, 2, false>(b, smem) : launch_tick<16, 1, false>(b, smem);
-    default: return u2 ? launch_tick<32, 2, false>(b, smem) : launch_tick<32, 1, false>(b, smem);
+    case 4: return u2 ? launch_tick<8, 2>(b, smem) : launch_tick<8, 1>(b, smem);
+    case 2: return u2 ? launch_tick<16, 2>(b, smem) : launch_tick<16, 1>(b, smem);
+    default: return u2 ? launch_tick<32, 2>(b, smem) : launch_tick<32, 1>(b, smem);
   }
 }
 
-// Enqueues one tick: parameters up, the persistent kernel, results back.
-cudaError_t enqueue_tick(bxg_batch b, size_t param_bytes, size_t smem, bool mark) {
+cudaError_t launch_two_phase(bxg_batch b, bool tail) {
+  const TickArgs* a = b->params.as<TickArgs>();
+  const TickScan* s = reinterpret_cast<const TickScan*>(b->params.as<uint8_t>() + 256);
+  const unsigned wave = unsigned(b->sm_count) * 8;
+  k_tick_begin<<<wave, 256, 0, b->stream>>>(a, s);
+  k_tick_endpoints<<<wave, 256, 0, b->stream>>>(a, s);
+  k_tick_winners<<<wave, 256, 0, b->stream>>>(a, s);
+  k_tick_mark<<<b->grid_mark, kMarkThreads, 0, b->stream>>>(a, s);
+  k_tick_roots<<<b->sm_count, 256, 0, b->stream>>>(a, s);
+  k_tick_apply<<<b->sm_count * 32, 256, 0, b->stream>>>(a, s);
+  if (tail) k_tick_tail<<<wave, 256, 0, b->stream>>>(a, s);
+  k_tick_end<<<(kMaxTickScans * C_WORDS + 255) / 256, 256, 0, b->stream>>>(a, s);
+  return cudaGetLastError();
+}
+
+// Enqueues one tick: parameters up, the kernels, results back.
+cudaError_t enqueue_tick(bxg_batch b, size_t param_bytes, size_t smem, bool mark, bool tail) {
   cudaError_t e = cudaMemcpyAsync(b->params.p, b->h_args, param_bytes, cudaMemcpyHostToDevice,
                                   b->stream);
   if (e != cudaSuccess) return e;
   e = cudaMemsetAsync(b->meta.p, 0, 16, b->stream);  // barrier, error and ray-counter words
   if (e != cudaSuccess) return e;
-  e = launch_for(b, smem, mark);
+  e = mark ? launch_two_phase(b, tail) : launch_single_pass(b, smem);
   if (e != cudaSuccess) return e;
   return cudaMemcpyAsync(b->h_back, b->meta.p, kBackBytes, cudaMemcpyDeviceToHost, b->stream);
 }
@@ -556,15 +700,14 @@ int bxg_batch_create(bxg_batch* out, const bxg_config* cfg_in) {
     delete b;
     return BXG_ERR_CUDA;
   }
-  const int smem = int(tick_smem(false, kMaxTickScans));
-  cudaFuncSetAttribute(k_tick<32, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  cudaFuncSetAttribute(k_tick<16, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  cudaFuncSetAttribute(k_tick<8, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  cudaFuncSetAttribute(k_tick<32, 2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  cudaFuncSetAttribute(k_tick<16, 2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  cudaFuncSetAttribute(k_tick<8, 2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  cudaFuncSetAttribute(k_tick<32, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       int(tick_smem(true, kMaxTickScans)));
+  const int smem = int(tick_smem(kMaxTickScans));
+  cudaFuncSetAttribute(k_tick<32, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  cudaFuncSetAttribute(k_tick<16, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  cudaFuncSetAttribute(k_tick<8, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  cudaFuncSetAttribute(k_tick<32, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  cudaFuncSetAttribute(k_tick<16, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  cudaFuncSetAttribute(k_tick<8, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  b->grid_mark = b->sm_count * kMarkBlocksPerSM;
   cudaGetLastError();
   const size_t pbytes = 256 + kMaxTickScans * sizeof(TickScan);
   if (cudaMallocHost(reinterpret_cast<void**>(&b->h_args), pbytes) != cudaSuccess ||
@@ -659,8 +802,7 @@ int bxg_batch_insert_f32(bxg_batch b, const bxg_pmap* maps, size_t n_scans, cons
   A.ctr_out = reinterpret_cast<uint32_t*>(meta + kOffCtr);
   A.times = reinterpret_cast<unsigned long long*>(meta + kOffTime);
   A.ray_prefix = reinterpret_cast<uint32_t*>(meta + kOffPrefix);
-  A.task_prefix = reinterpret_cast<uint32_t*>(meta + kOffTaskPrefix);
-  A.chunk = reinterpret_cast<uint32_t*>(meta + kOffChunk);
+  A.n_roots = reinterpret_cast<uint32_t*>(meta + kOffRoots);
   A.n_scans = uint32_t(n_scans);
   A.total_points = total;
   A.total_tab = tab_total;
@@ -693,53 +835,58 @@ int bxg_batch_insert_f32(bxg_batch b, const bxg_pmap* maps, size_t n_scans, cons
   }
   // The two-phase ray update when every map can have its cube bitmap (each
   // map's own buffers, zero between scans; growing them synchronises the map).
-  bool mark = true;
+  bool mark = true, tail = false;
+  A.n_chunks = 0;
+  A.root_words = 0;
+  uint64_t seg_room = 0, root_room = 0;
+  std::vector<uint64_t> seg0(n_scans);
   for (size_t s = 0; s < n_scans && mark; s++) {
     TickScan& S = b->h_scans[s];
     bool ok = false;
-    const int st = cube_for_scan(maps[s], S.ox, S.oy, S.oz, S.max_range, &S.Q, &ok);
+    const int st = scan_cube(maps[s], S.ox, S.oy, S.oz, S.max_range, 0, &S.Q, &ok);
     if (st) return bfail(b, st, maps[s]->core.err);
     mark = ok;
-  }
-  // the list phase's index space: 32 touched words per chunk, scan after scan
-  A.n_chunks = 0;
-  for (size_t s = 0; s < n_scans && mark; s++) {
-    TickScan& S = b->h_scans[s];
+    if (!ok) break;
+    tail |= S.Q.open != 0;
     S.chunk0 = A.n_chunks;
-    A.n_chunks += (cube_touched_words(S.Q) + 31u) / 32u;
+    A.n_chunks += (S.n + 255u) / 256u;
+    S.root0 = A.root_words;
+    A.root_words += cube_root_words(S.Q);
+    root_room += uint64_t(S.Q.SR) * S.Q.SR * S.Q.SR;
+    seg0[s] = seg_room;
+    // a segment is a ray's position (24 bits) and a number (8 bits)
+    if (S.n <= (1u << 24)) seg_room += uint64_t(S.n) * max_segments(S.Q);
   }
-  // each map's kept leaf directory for the apply phase (its memsets go on the
-  // batch's stream, ahead of the tick)
-  for (size_t s = 0; s < n_scans && mark; s++) {
-    TickScan& S = b->h_scans[s];
-    maps[s]->dir_reach = S.max_range;
-    const int st = leaf_dir_for_scan(maps[s], S.ox, S.oy, S.oz, &S.D, size_t(1) << 23, b->stream);
-    maps[s]->dir_reach = 0.0;
-    if (st) return bfail(b, st, maps[s]->core.err);
+  if (mark) {
+    BB_CUDA(b, grow(b->segs, seg_room * 4 + 16));
+    BB_CUDA(b, grow(b->roots, root_room * 4 + 16));
+    if (tail) BB_CUDA(b, grow(b->tails, total * 4 + 16));
+    A.roots = b->roots.as<uint32_t>();
+    for (size_t s = 0; s < n_scans; s++) {
+      TickScan& S = b->h_scans[s];
+      if (S.n <= (1u << 24)) S.Q.segs = b->segs.as<uint32_t>() + seg0[s];
+      if (S.Q.open) S.Q.tails = b->tails.as<uint32_t>() + S.pt_begin;
+    }
   }
   b->back_bytes = kBackBytes;
   const size_t param_bytes = 256 + n_scans * sizeof(TickScan);
-  const size_t smem = tick_smem(mark, n_scans);
+  const size_t smem = tick_smem(n_scans);
   // resident blocks for this shared-memory size (the launch is cooperative)
-  if (mark && (!b->grid_mark || b->grid_smem[1] != smem)) {
-    b->grid_mark = occupancy_grid<32, 1, true>(b, smem);
-    b->grid_smem[1] = smem;
-    if (b->grid_mark <= 0) return bfail(b, BXG_ERR_CUDA, "k_tick cannot be resident");
-  } else if (!mark && (!b->grid || b->grid_smem[0] != smem)) {
+  if (!mark && (!b->grid || b->grid_smem != smem)) {
     const bool u2 = b->ray_unroll == 2;
     switch (b->rays_per_warp) {
-      case 4: b->grid = u2 ? occupancy_grid<8, 2, false>(b, smem) : occupancy_grid<8, 1, false>(b, smem); break;
-      case 2: b->grid = u2 ? occupancy_grid<16, 2, false>(b, smem) : occupancy_grid<16, 1, false>(b, smem); break;
-      default: b->grid = u2 ? occupancy_grid<32, 2, false>(b, smem) : occupancy_grid<32, 1, false>(b, smem); break;
+      case 4: b->grid = u2 ? occupancy_grid<8, 2>(b, smem) : occupancy_grid<8, 1>(b, smem); break;
+      case 2: b->grid = u2 ? occupancy_grid<16, 2>(b, smem) : occupancy_grid<16, 1>(b, smem); break;
+      default: b->grid = u2 ? occupancy_grid<32, 2>(b, smem) : occupancy_grid<32, 1>(b, smem); break;
     }
-    b->grid_smem[0] = smem;
+    b->grid_smem = smem;
     if (b->grid <= 0) return bfail(b, BXG_ERR_CUDA, "k_tick cannot be resident");
   }
 
   // Run: the captured graph when its shape matches, else capture it again.
-  const uint64_t key[7] = {uint64_t(b->params.p), param_bytes, uint64_t(b->meta.p), b->back_bytes,
+  const uint64_t key[8] = {uint64_t(b->params.p), param_bytes, uint64_t(b->meta.p), b->back_bytes,
                            uint64_t(mark ? b->grid_mark : b->grid), b->rays_per_warp,
-                           mark ? 1ull : 0ull};
+                           mark ? 1ull : 0ull, tail ? 1ull : 0ull};
   cudaEventRecord(b->ev0, b->stream);
   bool ran = false;
   if (b->use_graph) {
@@ -750,7 +897,7 @@ int bxg_batch_insert_f32(bxg_batch b, const bxg_pmap* maps, size_t n_scans, cons
       b->graph = nullptr;
       b->graph_ok = false;
       if (cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
-        const cudaError_t e1 = enqueue_tick(b, param_bytes, smem, mark);
+        const cudaError_t e1 = enqueue_tick(b, param_bytes, smem, mark, tail);
         const cudaError_t e2 = cudaStreamEndCapture(b->stream, &b->graph);
         if (e1 == cudaSuccess && e2 == cudaSuccess &&
             cudaGraphInstantiate(&b->exec, b->graph, 0) == cudaSuccess) {
@@ -765,7 +912,7 @@ int bxg_batch_insert_f32(bxg_batch b, const bxg_pmap* maps, size_t n_scans, cons
       ran = true;
     }
   }
-  if (!ran) BB_CUDA(b, enqueue_tick(b, param_bytes, smem, mark));
+  if (!ran) BB_CUDA(b, enqueue_tick(b, param_bytes, smem, mark, tail));
   cudaEventRecord(b->ev1, b->stream);
   BB_CUDA(b, cudaStreamSynchronize(b->stream));
   b->launches++;
@@ -777,7 +924,12 @@ int bxg_batch_insert_f32(bxg_batch b, const bxg_pmap* maps, size_t n_scans, cons
     return bfail(b, BXG_ERR_WAIT_TIMEOUT, "a grid barrier timed out");
   {
     const unsigned long long* ts = reinterpret_cast<const unsigned long long*>(b->h_back + kOffTime);
-    for (int k = 0; k < 5; k++) b->phase_ms[k] = double(ts[k + 1] - ts[k]) * 1e-6;
+    for (int k = 0; k < 5; k++)
+      if (!mark || (k != 2 && k != 3)) b->phase_ms[k] = double(ts[k + 1] - ts[k]) * 1e-6;
+    if (mark) {  // winners end where mark begins; there is no prefix phase
+      b->phase_ms[2] = double(ts[4] - ts[2]) * 1e-6;
+      b->phase_ms[3] = 0.0;
+    }
     b->phase_ms[5] = mark ? double(ts[6] - ts[4]) * 1e-6 : 0.0;
   }
   const unsigned long long* stats =
@@ -792,12 +944,16 @@ int bxg_batch_insert_f32(bxg_batch b, const bxg_pmap* maps, size_t n_scans, cons
     const uint32_t prev_leaves = m->h_ctr[C_LEAF];
     std::memcpy(m->h_ctr, ctr + s * C_WORDS, C_WORDS * 4);
     m->dm.has_free = m->h_ctr[C_FREE_LEAF] > 0 ? 1u : 0u;
+    const unsigned long long* hs =
+        mark ? reinterpret_cast<const unsigned long long*>(m->h_ctr + C_STATS) : stats + 4 * s;
+    const unsigned long long st4[4] = {hs[S_POINTS], hs[S_RAY_LEN], hs[S_VISITED], hs[S_UPDATED]};
+    const uint32_t rays = mark ? m->h_ctr[C_CAST] : cnt[s];
     const uint32_t e = m->h_ctr[C_ERR];
     if (e & (ERR_POOL_INNER | ERR_POOL_LEAF | ERR_HASH_FULL)) {
       b->last_retries++;
       const TickScan& S = b->h_scans[s];
       const int st = pmap_complete_scan(pm, b->cast.as<int4>() + S.pt_begin,
-                                        A.cast_cnt + s, S.n, S.ox, S.oy, S.oz, S.u);
+                                        mark ? S.M.ctr + C_CAST : A.cast_cnt + s, S.n, S.ox, S.oy, S.oz, S.u);
       if (st && !status) {
         status = st;
         b->err = m->err;
@@ -810,12 +966,12 @@ int bxg_batch_insert_f32(bxg_batch b, const bxg_pmap* maps, size_t n_scans, cons
       }
     }
     pm->last_new_leaves = m->h_ctr[C_LEAF] > prev_leaves ? m->h_ctr[C_LEAF] - prev_leaves : 0;
-    pm->last_stats[0] = stats[4 * s + 0];
-    pm->last_stats[1] = cnt[s];
-    pm->last_stats[2] = stats[4 * s + 2];
-    pm->last_stats[3] = stats[4 * s + 3];
+    pm->last_stats[0] = st4[0];
+    pm->last_stats[1] = rays;
+    pm->last_stats[2] = st4[2];
+    pm->last_stats[3] = st4[3];
     pm->last_stats[4] = m->h_ctr[C_LEAF];
-    if (ray_cells) ray_cells[s] = stats[4 * s + 0] + stats[4 * s + 1];
+    if (ray_cells) ray_cells[s] = st4[0] + st4[1];
     if (++pm->update_count == 4) pm->update_count = 1;
   }
   return status;
@@ -833,7 +989,7 @@ int bxg_batch_stats(bxg_batch b, double out[8]) {
   out[1] = b->graph_ok ? 1 : 0;
   out[2] = double(b->last_retries);
   out[3] = double(b->ticks);
-  out[4] = double(b->grid_mark ? b->grid_mark : b->grid);
+  out[4] = double(b->grid ? b->grid : b->grid_mark);
   out[5] = double(b->launches);
   out[6] = b->phase_ms[1];  // endpoints
   out[7] = b->phase_ms[2] + b->phase_ms[4];  // winners + rays

@@ -185,11 +185,11 @@ struct bxg_pmap_s {
   uint32_t dir_epoch = 0;
   uint64_t dir_gen = 0;
   bool dir_live = false;
-  // the ray phase's cube bitmap, list bits and list (bxg_mark.cuh): all zero
-  // between scans; sized for cube_blocks leaf blocks
-  bxg::DevBuf cube_bits, cube_touch, cube_list;
+  // the ray phase's cube bitmap (bxg_mark.cuh): all zero between scans, sized for
+  // cube_blocks leaf blocks; root bits of the marked cells; and, of the per-map
+  // path, the rays' segments and the rays that leave the cube
+  bxg::DevBuf cube_bits;
   size_t cube_blocks = 0;
-  // root bits of the marked cells and the rays' segments, of the per-scan form
   bxg::DevBuf cube_roots, ray_segs, ray_tails;
   bool has_segs = false;  // the ray list's segments are in ray_segs, long rays in ray_tails
   cudaEvent_t ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
@@ -208,15 +208,8 @@ namespace bxg {
 // Buffers grow here (cudaMalloc, zeroed).
 int scan_cube(bxg_pmap_s* pm, int ox, int oy, int oz, double reach, uint64_t rays, ScanCube* Q,
               bool* ok);
-// The cube bitmap of a scan's ray phase from origin cell (ox, oy, oz) whose
-// rays end within `reach` (world units) of the origin: *ok = false when the
-// scan cannot use one (leaf_bits other than 3, non-finite points kept, a cube
-// above the size limit); buffers grow here (cudaMalloc, zeroed).
-int cube_for_scan(bxg_pmap_s* pm, int ox, int oy, int oz, double reach, RayCube* Q, bool* ok);
 // Sets up the ray walk's leaf directory of a scan (bxg_pmap.cu).
-// Memsets (first use, epoch wrap) go to `stream` (nullptr: the map's own).
-int leaf_dir_for_scan(bxg_pmap_s* pm, int ox, int oy, int oz, LeafDir* D, size_t max_words,
-                      cudaStream_t stream);
+int leaf_dir_for_scan(bxg_pmap_s* pm, int ox, int oy, int oz, LeafDir* D, size_t max_words);
 // Completes a scan whose endpoints were listed (and possibly applied) by a
 // batched tick but whose map ran out of pool: grows the pools and re-runs the
 // idempotent endpoint completion and ray phases on the map's own stream.

@@ -47,7 +47,7 @@ __device__ __forceinline__ void zero_scan_stats(const DMap& M, int zero,
        t += gridDim.x * blockDim.x)
     roots[t] = 0u;
   if (blockIdx.x != 0) return;
-  if ((zero & ZERO_RAYS) && threadIdx.x == 33) M.ctr[C_SEGS] = M.ctr[C_LIST] = 0u;
+  if ((zero & ZERO_RAYS) && threadIdx.x == 33) M.ctr[C_SEGS] = M.ctr[C_TAILS] = 0u;
   if ((zero & ZERO_STATS) && threadIdx.x < S_COUNT)
     reinterpret_cast<unsigned long long*>(M.ctr + C_STATS)[threadIdx.x] = 0ull;
   if ((zero & ZERO_CAST) && threadIdx.x == 32) M.ctr[C_CAST] = 0u;
@@ -66,16 +66,7 @@ __global__ void k_endpoints(const __grid_constant__ DMap M, const uint8_t* __res
     const PT* p = reinterpret_cast<const PT*>(pts + size_t(i) * stride);
     e = compute_endpoint<PT>(p, fx, fy, fz, max_range, mr2, inv_res, keep_nonfinite != 0, &F);
   }
-  // Neighbouring points often share an endpoint cell: within a warp only the
-  // lowest lane (lowest index) of each cell enters the table; the others can
-  // never be the cell's lowest index and are marked EP_DUP.
-  const unsigned vm = __ballot_sync(0xffffffffu, e.w != EP_SKIP);
-  if (e.w != EP_SKIP) {
-    const unsigned same = __match_any_sync(vm, e.x) & __match_any_sync(vm, e.y) &
-                          __match_any_sync(vm, e.z);
-    if (same & ((1u << (threadIdx.x & 31)) - 1u)) e.w = EP_DUP;
-    else dedup_min_insert(tab, tmask, e.x, e.y, e.z, i, M);
-  }
+  endpoint_enter(M, e, i, tab, tmask);
   if (i < n) ep[i] = e;
 }
 
@@ -133,93 +124,14 @@ __global__ void k_endpoints_kind(const __grid_constant__ DMap M, const double* _
   dedup_min_insert(tab, tmask, cx, cy, cz, i, M);
 }
 
-// The lowest-index point of each endpoint cell decides and applies
-// (winner_apply) and, if its ray is cast, joins the ray list.
-// One block-wide atomic each for the ray list, the point count and the ray
-// lengths (a per-warp atomic on three shared counters serialised in L2).
+// The lowest-index point of each endpoint cell (winners_block).
 __global__ void __launch_bounds__(256) k_winners(const __grid_constant__ DMap M, const int4* __restrict__ ep, uint32_t n,
                           const uint4* __restrict__ tab, uint32_t tmask, int ox, int oy, int oz,
                           int32_t u, Opts o, int4* __restrict__ cast, uint32_t cast_cap,
                           const __grid_constant__ ScanCube Q) {
-  __shared__ uint32_t s_cnt[8], s_pts[8], s_base, s_seg[8], s_seg_base, s_tail[8], s_tail_base;
-  __shared__ unsigned long long s_len[8];
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  bool add = false;
-  int4 e = make_int4(0, 0, 0, EP_SKIP);
-  if (i < n) {
-    e = ep[i];
-    if (e.w == EP_HIT || e.w == EP_MISS) {
-      if (dedup_lookup(tab, tmask, e.x, e.y, e.z) == i) add = winner_apply(M, e, u, o);
-    }
-  }
-  const unsigned lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const unsigned valid = __ballot_sync(0xffffffffu, i < n && e.w != EP_SKIP);
-  const unsigned am = __ballot_sync(0xffffffffu, add);
-  const uint32_t len = add ? chebyshev(ox, oy, oz, e.x, e.y, e.z) : 0u;
-  const unsigned long long wlen = __reduce_add_sync(0xffffffffu, len >> 16) * 65536ull +
-                                  __reduce_add_sync(0xffffffffu, len & 0xFFFFu);
-  // with a cube, the ray's segments go on the scan's list of segments
-  const uint32_t nseg = add && Q.segs ? far_segments(Q, len) : 0u;
-  uint32_t seg = nseg;
-#pragma unroll
-  for (int o2 = 1; o2 < 32; o2 <<= 1) {
-    const uint32_t v = __shfl_up_sync(0xffffffffu, seg, o2);
-    if (lane >= unsigned(o2)) seg += v;
-  }
-  if (lane == 31) s_seg[wid] = seg;
-  // and the rays that leave the cube on the list of those
-  const unsigned tails =
-      __ballot_sync(0xffffffffu, add && Q.tails && len > Q.kin);
-  if (lane == 0) {
-    s_cnt[wid] = __popc(am);
-    s_tail[wid] = __popc(tails);
-    s_pts[wid] = __popc(valid);
-    s_len[wid] = wlen;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    uint32_t tot = 0, pts = 0, segs = 0, tl_n = 0;
-    unsigned long long tl = 0;
-    for (unsigned w = 0; w < blockDim.x / 32; w++) {
-      const uint32_t c = s_cnt[w];
-      s_cnt[w] = tot;
-      tot += c;
-      pts += s_pts[w];
-      tl += s_len[w];
-      const uint32_t g = s_seg[w];
-      s_seg[w] = segs;
-      segs += g;
-      const uint32_t r = s_tail[w];
-      s_tail[w] = tl_n;
-      tl_n += r;
-    }
-    s_tail_base = tl_n ? atomicAdd(M.ctr + C_LIST, tl_n) : 0u;
-    s_seg_base = segs ? atomicAdd(M.ctr + C_SEGS, segs) : 0u;
-    unsigned long long* st = reinterpret_cast<unsigned long long*>(M.ctr + C_STATS);
-    if (pts) atomicAdd(st + S_POINTS, static_cast<unsigned long long>(pts));
-    if (tl) atomicAdd(st + S_RAY_LEN, tl);
-    s_base = tot ? atomicAdd(M.ctr + C_CAST, tot) : 0u;
-  }
-  __syncthreads();
-  uint32_t s_k = 0;
-  if (add) {
-    const uint32_t k = s_base + s_cnt[wid] + __popc(am & ((1u << lane) - 1));
-    if (k < cast_cap)
-      cast[k] = e;
-    else
-      set_err(M, ERR_SCRATCH);
-    s_k = k;
-    if ((tails >> lane) & 1u)
-      Q.tails[s_tail_base + s_tail[wid] + __popc(tails & ((1u << lane) - 1u))] = k;
-  }
-  // the warp's segments, number by number: neighbouring rays' segments lie side by side
-  uint32_t at = s_seg_base + s_seg[wid];
-  for (uint32_t j = 0;; ++j) {
-    const unsigned has = __ballot_sync(0xffffffffu, nseg > j);
-    if (!has) break;
-    if (nseg > j) Q.segs[at + __popc(has & ((1u << lane) - 1u))] = (s_k << 8) | j;
-    at += __popc(has);
-  }
+  __shared__ WinnersShared S;
+  winners_block(M, ep, n, blockIdx.x * blockDim.x + threadIdx.x, tab, tmask, ox, oy, oz, u, o,
+                cast, cast_cap, Q, S);
 }
 
 // Completes listed endpoints after a pool ran out: creates each cell and
@@ -293,7 +205,9 @@ __global__ void __launch_bounds__(kMarkThreads, kMarkBlocksPerSM) k_mark(
   const uint32_t n_cast = min(ld_volatile(M.ctr + C_CAST), cast_cap);
   const uint32_t n_segs = ld_volatile(M.ctr + C_SEGS);
   uint32_t visited = 0;
-  mark_scan(M, Q, cast, n_cast, n_segs, blockIdx.x, gridDim.x, ox, oy, oz, S, visited);
+  const uint32_t first = blockIdx.x * kMarkThreads;
+  mark_scan(M, Q, cast, first, n_cast, first, Q.segs ? n_segs : 0u, gridDim.x * kMarkThreads, ox,
+            oy, oz, S, visited);
   visited = __reduce_add_sync(0xffffffffu, visited);
   if ((threadIdx.x & 31) == 0 && visited)
     atomicAdd(reinterpret_cast<unsigned long long*>(M.ctr + C_STATS) + S_VISITED,
@@ -304,58 +218,29 @@ __global__ void __launch_bounds__(kMarkThreads, kMarkBlocksPerSM) k_mark(
 __global__ void __launch_bounds__(256, 6) k_apply_rays(const __grid_constant__ DMap M,
                                                     const __grid_constant__ ScanCube Q, int32_t u,
                                                     int32_t miss, int32_t cmin) {
-  __shared__ uint32_t pre[kRootFlagWords], sums[8];
+  __shared__ uint32_t pre[kRootFlagWords], sums[kApplyWarps];
+  __shared__ ApplyShared S;
   const uint32_t n_roots = apply_roots(Q, pre, sums);
   const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   uint32_t updated = 0;
-  apply_scan(M, Q, n_roots, pre, gw, (gridDim.x * blockDim.x) >> 5, u, miss, cmin, updated);
+  apply_scan(M, Q, n_roots, pre, gw, (gridDim.x * blockDim.x) >> 5, u, miss, cmin,
+             S.rows[threadIdx.x >> 5], updated);
   updated = __reduce_add_sync(0xffffffffu, updated);
   if ((threadIdx.x & 31) == 0 && updated)
     atomicAdd(reinterpret_cast<unsigned long long*>(M.ctr + C_STATS) + S_UPDATED,
               static_cast<unsigned long long>(updated));
 }
 
-// The parts of rays that the cube does not hold (cells k >= kin; all cells of a
-// ray of kMarkMaxRay cells or more), walked on the tree. A warp takes a piece of a
-// ray, 1 / kTailPieces of it and at least two steps of 32 cells: a walk is a
-// chain of dependent loads, about 4 us a step, and the rays that go far are few
-// (29 k points at 0.05 m with returns to 100 m: 16 us; with eight rays per warp and
-// pieces of 256 cells 125 us; the whole scan walked by k_rays 330 us, against 17
-// for k_mark, 25 for k_apply_rays and this). Without a list of them (rays queued
-// by addHitPoint/addMissPoint) all rays are looked at.
-constexpr uint32_t kTailPieces = 32;
+// The parts of the scan's rays that the cube does not hold (tail_rays).
 __global__ void __launch_bounds__(256) k_tail(const __grid_constant__ DMap M,
                                               const __grid_constant__ ScanCube Q,
                                               const int4* __restrict__ cast, uint32_t cast_cap,
                                               int ox, int oy, int oz, int32_t u, int32_t miss,
                                               int32_t cmin) {
-  const uint32_t n = Q.tails ? ld_volatile(M.ctr + C_LIST) : min(ld_volatile(M.ctr + C_CAST), cast_cap);
-  const unsigned lane = threadIdx.x & 31;
-  const uint64_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint64_t nw = (gridDim.x * blockDim.x) >> 5;
   uint32_t visited = 0, updated = 0;
-  for (uint64_t t = gw; t < uint64_t(n) * kTailPieces; t += nw) {
-    const uint32_t i = uint32_t(t / kTailPieces), j = uint32_t(t % kTailPieces);
-    const int4 e = cast[Q.tails ? Q.tails[i] : i];
-    const uint32_t m = chebyshev(ox, oy, oz, e.x, e.y, e.z);
-    if (m <= Q.kin) continue;
-    if (m >= kMaxRayCells) {
-      if (lane == 0) set_err(M, ERR_RAY_TOO_LONG);
-      continue;
-    }
-    const uint32_t from = m < kMarkMaxRay ? Q.kin : 0u;
-    const uint32_t piece = max(64u, (((m - from) / kTailPieces + 32u) & ~31u));
-    if (from + j * piece < m)
-      walk_ray<32>(M, e, ox, oy, oz, u, miss, cmin, lane, 0u, 0xffffffffu, visited, updated,
-                   nullptr, from + j * piece, from + (j + 1) * piece);
-  }
-  visited = __reduce_add_sync(0xffffffffu, visited);
-  updated = __reduce_add_sync(0xffffffffu, updated);
-  if (lane == 0 && visited) {
-    unsigned long long* st = reinterpret_cast<unsigned long long*>(M.ctr + C_STATS);
-    atomicAdd(st + S_VISITED, static_cast<unsigned long long>(visited));
-    atomicAdd(st + S_UPDATED, static_cast<unsigned long long>(updated));
-  }
+  tail_rays(M, Q, cast, cast_cap, (blockIdx.x * blockDim.x + threadIdx.x) >> 5,
+            (gridDim.x * blockDim.x) >> 5, ox, oy, oz, u, miss, cmin, visited, updated);
+  tail_count(M, visited, updated);
 }
 
 // isOccupied / isUnknown / isFree (probabilistic_map.cpp:56-75).
@@ -505,10 +390,8 @@ namespace bxg {
 // the 4-bit epoch wraps, so a word of another epoch is always empty. *D stays
 // empty (the walk probes the root hash for every leaf run) when the cube would
 // exceed max_words words or leaf slots do not fit in 28 bits.
-int leaf_dir_for_scan(bxg_pmap_s* pm, int ox, int oy, int oz, LeafDir* D, size_t max_words,
-                      cudaStream_t stream) {
+int leaf_dir_for_scan(bxg_pmap_s* pm, int ox, int oy, int oz, LeafDir* D, size_t max_words) {
   MapCore* m = &pm->core;
-  if (!stream) stream = m->stream;
   *D = LeafDir{};
   if (!(pm->dir_reach > 0) || m->dm.lcap >= (1u << 28)) return BXG_OK;
   const double cells = std::ceil(pm->dir_reach * m->inv_res) + 2;
@@ -528,11 +411,11 @@ int leaf_dir_for_scan(bxg_pmap_s* pm, int ox, int oy, int oz, LeafDir* D, size_t
     const size_t words = words_of(h);
     if (m->s_dir.cap < words * 4) {
       BXG_CUDA(m, m->s_dir.ensure(words * 4));
-      BXG_CUDA(m, cudaMemsetAsync(m->s_dir.p, 0, m->s_dir.cap, stream));
+      BXG_CUDA(m, cudaMemsetAsync(m->s_dir.p, 0, m->s_dir.cap, m->stream));
       pm->dir_epoch = 0;
     }
     if (++pm->dir_epoch == 16) {  // the epoch wraps: clear every word ever written
-      BXG_CUDA(m, cudaMemsetAsync(m->s_dir.p, 0, m->s_dir.cap, stream));
+      BXG_CUDA(m, cudaMemsetAsync(m->s_dir.p, 0, m->s_dir.cap, m->stream));
       pm->dir_epoch = 1;
     }
     pm->dir_x0 = cx - h;
@@ -577,16 +460,14 @@ int scan_cube(bxg_pmap_s* pm, int ox, int oy, int oz, double reach, uint64_t ray
   if (blocks > pm->cube_blocks) {
     BXG_CUDA(m, pm->cube_bits.ensure(blocks * 64));
     BXG_CUDA(m, cudaMemsetAsync(pm->cube_bits.p, 0, pm->cube_bits.cap, m->stream));
-    // the batched tick uses the buffers from another stream
-    BXG_CUDA(m, cudaStreamSynchronize(m->stream));
     pm->cube_blocks = blocks;
-  }
-  if (!pm->cube_roots.p) {
     BXG_CUDA(m, pm->cube_roots.ensure(kRootFlagWords * 4));
     BXG_CUDA(m, cudaMemsetAsync(pm->cube_roots.p, 0, pm->cube_roots.cap, m->stream));
+    // the batched tick uses the buffers from another stream
+    BXG_CUDA(m, cudaStreamSynchronize(m->stream));
   }
   // a segment is a ray's position (24 bits) and a number (8 bits)
-  const uint64_t segs = rays * ((Q->kin - kNearCells + kSegCells - 1) / kSegCells);
+  const uint64_t segs = rays * max_segments(*Q);
   if (rays && rays <= (1u << 24) && segs <= (1u << 28)) {
     BXG_CUDA(m, pm->ray_segs.ensure(segs * 4));
     Q->segs = pm->ray_segs.as<uint32_t>();
@@ -600,54 +481,6 @@ int scan_cube(bxg_pmap_s* pm, int ox, int oy, int oz, double reach, uint64_t ray
   Q->x0 = ((ox >> 5) - h) * 32;
   Q->y0 = ((oy >> 5) - h) * 32;
   Q->z0 = ((oz >> 5) - h) * 32;
-  *ok = true;
-  return BXG_OK;
-}
-
-// Largest cube side (leaves): 200^3 blocks of 64 B = 512 MB of bits. Scans
-// whose cube would be larger (very fine resolutions with long ranges) walk
-// their rays with k_rays instead.
-constexpr uint32_t kMaxCubeSide = 200;
-
-int cube_for_scan(bxg_pmap_s* pm, int ox, int oy, int oz, double reach, RayCube* Q, bool* ok) {
-  MapCore* m = &pm->core;
-  *ok = false;
-  if (m->dm.lb != 3 || m->dm.esz != 4 ||
-      (m->flags & (BXG_FLAG_KEEP_NONFINITE | BXG_FLAG_RAYS_SINGLE_PASS)))
-    return BXG_OK;
-  if (!(reach > 0) || !std::isfinite(reach)) return BXG_OK;
-  // Ray ends lie within ceil(reach / res) + 2 cells of the origin cell (the
-  // floor of the origin and of the end each move a cell by less than one), so
-  // every ray cell lies within HL leaves of the origin's leaf.
-  const double cells = std::ceil(reach * m->inv_res) + 2.0;
-  if (!(cells < 8.0 * kMaxCubeSide)) return BXG_OK;
-  const int R = int(cells);
-  const int HL = std::max((R + 7) / 8 + 1, kMarkNB + 1);
-  const uint32_t S = uint32_t(2 * HL + 1);
-  if (S > kMaxCubeSide) return BXG_OK;
-  const size_t blocks = size_t(S) * S * S;
-  const uint32_t tmask = cube_touched_mask(S);
-  if (blocks > pm->cube_blocks || !pm->cube_touch.p ||
-      pm->cube_list.cap < blocks * 4 || pm->cube_touch.cap < (size_t(tmask) + 1) / 8) {
-    BXG_CUDA(m, pm->cube_bits.ensure(blocks * 64));
-    BXG_CUDA(m, pm->cube_touch.ensure((size_t(tmask) + 1) / 8));
-    BXG_CUDA(m, pm->cube_list.ensure(blocks * 4));
-    BXG_CUDA(m, cudaMemsetAsync(pm->cube_bits.p, 0, pm->cube_bits.cap, m->stream));
-    BXG_CUDA(m, cudaMemsetAsync(pm->cube_touch.p, 0, pm->cube_touch.cap, m->stream));
-    // the batched tick uses the buffers from another stream
-    BXG_CUDA(m, cudaStreamSynchronize(m->stream));
-    pm->cube_blocks = std::max(pm->cube_blocks, blocks);
-  }
-  Q->bits = pm->cube_bits.as<uint32_t>();
-  Q->touched = pm->cube_touch.as<uint32_t>();
-  Q->list = pm->cube_list.as<uint32_t>();
-  Q->count = m->ctr.as<uint32_t>() + C_LIST;
-  Q->x0 = ((ox >> 3) - HL) * 8;
-  Q->y0 = ((oy >> 3) - HL) * 8;
-  Q->z0 = ((oz >> 3) - HL) * 8;
-  Q->S = S;
-  Q->cap = uint32_t(blocks);
-  Q->tmask = tmask;
   *ok = true;
   return BXG_OK;
 }
@@ -735,7 +568,7 @@ int launch_rays(bxg_pmap_s* pm, int ox, int oy, int oz) {
   const dim3 g{unsigned(blocks)}, b{unsigned(bs)};
   const uint32_t tab_n = m->dedup_used;
   LeafDir dir{};
-  int st = leaf_dir_for_scan(pm, ox, oy, oz, &dir, size_t(1) << 24, m->stream);
+  int st = leaf_dir_for_scan(pm, ox, oy, oz, &dir, size_t(1) << 24);
   if (st) return st;
   kern<<<g, b, 0, m->stream>>>(m->dm, m->s_cast.as<int4>(), ccap, ox, oy, oz, pm->update_count,
                                o.miss, o.cmin, m->s_dedup.as<uint4>(), tab_n, dir);
@@ -1080,8 +913,9 @@ int pmap_complete_scan(bxg_pmap_s* pm, const int4* d_cast, const uint32_t* d_cou
   if (st && (!(err & (ERR_POOL_INNER | ERR_POOL_LEAF | ERR_HASH_FULL)) ||
               (err & (ERR_WAIT | ERR_RAY_TOO_LONG | ERR_SCRATCH))))
     return st;
-  BXG_CUDA(m, cudaMemcpyAsync(m->ctr.as<uint32_t>() + C_CAST, d_count, 4,
-                              cudaMemcpyDeviceToDevice, m->stream));
+  if (d_count != m->ctr.as<uint32_t>() + C_CAST)
+    BXG_CUDA(m, cudaMemcpyAsync(m->ctr.as<uint32_t>() + C_CAST, d_count, 4,
+                                cudaMemcpyDeviceToDevice, m->stream));
   for (int attempt = 0; attempt < 12 && err; attempt++) {
     st = core_grow_for(m, err);
     if (st) return st;

@@ -340,7 +340,7 @@ bxg_grid bxg_pmap_grid(bxg_pmap m);
 /* ========================================================================
  * Batched scans: insertPointCloud (probabilistic_map.hpp:141-160) on many
  * independent maps at once -- one scan per map per call, all maps' phases in
- * one persistent launch replayed from a CUDA graph. Each map ends bit-identical
+ * a few launches replayed from a CUDA graph. Each map ends bit-identical
  * to inserting its scan alone; the maps must live on the batch's device and
  * have no rays queued by bxg_pmap_add_*_points.
  * ======================================================================== */
@@ -359,7 +359,8 @@ int bxg_batch_insert_f32(bxg_batch b, const bxg_pmap* maps, size_t n_scans, cons
                          const uint64_t* offsets, const float* origins, const double* max_ranges,
                          uint64_t* ray_cells);
 /* Last tick: [0] device ms, [1] ran as a CUDA graph, [2] maps completed after
- * a pool ran out, [3] ticks so far, [4] persistent grid (blocks), [5] tick
+ * a pool ran out, [3] ticks so far, [4] blocks of the mark phase (of the
+ * persistent kernel in the single-pass form), [5] tick
  * launches so far, [6] endpoint phase ms, [7] winner + ray phases ms. */
 int bxg_batch_stats(bxg_batch b, double out[8]);
 /* Last tick's phases in ms (device global timer): [0] clear, [1] endpoints,
