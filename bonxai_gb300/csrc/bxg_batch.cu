@@ -840,6 +840,7 @@ int bxg_batch_insert_f32(bxg_batch b, const bxg_pmap* maps, size_t n_scans, cons
   A.root_words = 0;
   uint64_t seg_room = 0, root_room = 0;
   std::vector<uint64_t> seg0(n_scans);
+  std::vector<char> has_segs(n_scans);
   for (size_t s = 0; s < n_scans && mark; s++) {
     TickScan& S = b->h_scans[s];
     bool ok = false;
@@ -854,8 +855,11 @@ int bxg_batch_insert_f32(bxg_batch b, const bxg_pmap* maps, size_t n_scans, cons
     A.root_words += cube_root_words(S.Q);
     root_room += uint64_t(S.Q.SR) * S.Q.SR * S.Q.SR;
     seg0[s] = seg_room;
-    // a segment is a ray's position (24 bits) and a number (8 bits)
-    if (S.n <= (1u << 24)) seg_room += uint64_t(S.n) * max_segments(S.Q);
+    // a segment is a ray's position (24 bits) and a number (8 bits); scans for which the
+    // lists of all scans would take more than 2 GB are walked ray by ray
+    const uint64_t need = uint64_t(S.n) * max_segments(S.Q);
+    has_segs[s] = S.n <= (1u << 24) && seg_room + need <= (1u << 29);
+    if (has_segs[s]) seg_room += need;
   }
   if (mark) {
     BB_CUDA(b, grow(b->segs, seg_room * 4 + 16));
@@ -864,7 +868,7 @@ int bxg_batch_insert_f32(bxg_batch b, const bxg_pmap* maps, size_t n_scans, cons
     A.roots = b->roots.as<uint32_t>();
     for (size_t s = 0; s < n_scans; s++) {
       TickScan& S = b->h_scans[s];
-      if (S.n <= (1u << 24)) S.Q.segs = b->segs.as<uint32_t>() + seg0[s];
+      if (has_segs[s]) S.Q.segs = b->segs.as<uint32_t>() + seg0[s];
       if (S.Q.open) S.Q.tails = b->tails.as<uint32_t>() + S.pt_begin;
     }
   }

@@ -787,58 +787,88 @@ int add_points(bxg_pmap m_, const double* xyz, size_t n, int kind,
 // each occupied cell (probability_log > thr, probabilistic_map.cpp:108-116)
 // becomes its corner position coordToPos(c) = double(c) * res
 // (bonxai.hpp:413-417), kept when min_z <= z <= max_z, narrowed to float
-// xyz (the PCLPoint the node publishes). One thread per leaf mask word; a
-// warp reserves its output range with one atomic. Order is unspecified, as
-// the reference's unordered_map order is.
-__global__ void k_export_occupied(const __grid_constant__ DMap M, uint32_t n_leaves, float* __restrict__ out, size_t cap,
+// xyz (the PCLPoint the node publishes). Order is unspecified, as the
+// reference's unordered_map order is. (A ProbabilisticMap's leaves are 8^3.)
+//
+// A lane looks at rows of 8 cells (one mask byte, one 32-byte sector, one z): two of each of
+// its warp's kExportLeaves leaves, all their mask bytes loaded at once; only the
+// words of on cells in rows of the band are read, and the block takes its output range
+// with one atomic. Bound by the latency of mask, then cells. 82 k leaves with 26 k occupied
+// cells: 29 us (134 us with a thread per mask word, up to 64 cells one after the other).
+constexpr int kExportLeaves = 2;  // per warp (1: the same; 4: 33 us, 8: 38 us)
+__global__ void __launch_bounds__(256) k_export_occupied(const __grid_constant__ DMap M, uint32_t n_leaves, float* __restrict__ out, size_t cap,
                                   unsigned long long* __restrict__ counter, int32_t thr,
                                   double res, double min_z, double max_z) {
-  const size_t t = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
-  const uint32_t leaf = static_cast<uint32_t>(t / M.lwords);
-  const uint32_t wi = static_cast<uint32_t>(t % M.lwords);
-  const int lm = (1 << M.lb) - 1;
-  unsigned long long w = 0;
-  int4 key = make_int4(0, 0, 0, -1);
-  if (leaf < n_leaves) {
-    key = M.lkey[leaf];
-    if (key.w != -1) w = M.lmask[static_cast<size_t>(leaf) * M.lwords + wi];
-  }
-  if (w) {
-    const int32_t* cells = reinterpret_cast<const int32_t*>(M.ldata) +
-                           static_cast<size_t>(leaf) * M.lsize + wi * 64;
-    unsigned long long f = 0, rest = w;
-    while (rest) {
-      const int b = __ffsll(static_cast<long long>(rest)) - 1;
-      rest &= rest - 1;
-      const uint32_t ci = wi * 64 + b;
-      const double pz = __dmul_rn(double(key.z | int((ci >> (2 * M.lb)) & lm)), res);
-      if (cell_prob(cells[b]) > thr && pz >= min_z && pz <= max_z) f |= 1ull << b;
+  __shared__ uint32_t s_cnt[8];
+  __shared__ unsigned long long s_base;
+  const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t leaf0 = (blockIdx.x * 8u + warp) * kExportLeaves;
+  const uint8_t* mask = reinterpret_cast<const uint8_t*>(M.lmask);
+  int4 key[kExportLeaves];
+  uint32_t on[kExportLeaves][2];
+#pragma unroll
+  for (int l = 0; l < kExportLeaves; ++l) {
+    key[l] = make_int4(0, 0, 0, -1);
+    on[l][0] = on[l][1] = 0u;
+    if (leaf0 + l < n_leaves) {
+      key[l] = M.lkey[leaf0 + l];
+      on[l][0] = mask[size_t(leaf0 + l) * 64u + lane];
+      on[l][1] = mask[size_t(leaf0 + l) * 64u + 32u + lane];
     }
-    w = f;
   }
-  const unsigned cnt = __popcll(w);
-  const unsigned lane = threadIdx.x & 31;
-  unsigned incl = cnt;
+  // occupied cells of the rows: eight bits each
+  uint32_t cnt = 0;
+#pragma unroll
+  for (int l = 0; l < kExportLeaves; ++l)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const double pz = __dmul_rn(double(key[l].z | int((lane >> 3) + 4 * h)), res);
+      uint32_t w = key[l].w != -1 && pz >= min_z && pz <= max_z ? on[l][h] : 0u;
+      if (w) {
+        const int4* c = reinterpret_cast<const int4*>(M.ldata) + size_t(leaf0 + l) * 128u +
+                        2u * (lane + 32u * h);
+        int4 v[2];
+        if (w & 0xFu) v[0] = c[0];
+        if (w & 0xF0u) v[1] = c[1];
+        const int32_t* x = reinterpret_cast<const int32_t*>(v);
+#pragma unroll
+        for (int b = 0; b < 8; ++b)
+          if (((w >> b) & 1u) && !(cell_prob(x[b]) > thr)) w &= ~(1u << b);
+      }
+      on[l][h] = w;
+      cnt += __popc(w);
+    }
+  uint32_t incl = cnt;
+#pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    const unsigned v = __shfl_up_sync(0xffffffffu, incl, o);
+    const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
     if (lane >= static_cast<unsigned>(o)) incl += v;
   }
-  const unsigned total = __shfl_sync(0xffffffffu, incl, 31);
-  unsigned long long base = 0;
-  if (lane == 31 && total) base = atomicAdd(counter, static_cast<unsigned long long>(total));
-  base = __shfl_sync(0xffffffffu, base, 31);
-  unsigned long long pos = base + incl - cnt;
-  while (w) {
-    const int b = __ffsll(static_cast<long long>(w)) - 1;
-    w &= w - 1;
-    const uint32_t ci = wi * 64 + b;
-    if (pos < cap) {
-      out[3 * pos + 0] = float(__dmul_rn(double(key.x | int(ci & lm)), res));
-      out[3 * pos + 1] = float(__dmul_rn(double(key.y | int((ci >> M.lb) & lm)), res));
-      out[3 * pos + 2] = float(__dmul_rn(double(key.z | int((ci >> (2 * M.lb)) & lm)), res));
-    }
-    pos++;
+  if (lane == 31) s_cnt[warp] = incl;
+  __syncthreads();
+  uint32_t before = incl - cnt, total = 0;
+#pragma unroll
+  for (unsigned w = 0; w < 8; ++w) {
+    if (w < warp) before += s_cnt[w];
+    total += s_cnt[w];
   }
+  if (!total) return;
+  if (threadIdx.x == 0) s_base = atomicAdd(counter, static_cast<unsigned long long>(total));
+  __syncthreads();
+  unsigned long long pos = s_base + before;
+#pragma unroll
+  for (int l = 0; l < kExportLeaves; ++l)
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      for (uint32_t w = on[l][h]; w; w &= w - 1u) {
+        const int b = __ffs(static_cast<int>(w)) - 1;
+        if (pos < cap) {
+          out[3 * pos + 0] = float(__dmul_rn(double(key[l].x | b), res));
+          out[3 * pos + 1] = float(__dmul_rn(double(key[l].y | int(lane & 7u)), res));
+          out[3 * pos + 2] = float(__dmul_rn(double(key[l].z | int((lane >> 3) + 4 * h)), res));
+        }
+        pos++;
+      }
 }
 
 int export_occupied(bxg_pmap m_, float* out_xyz, size_t cap, size_t* n_out, double min_z,
@@ -854,10 +884,10 @@ int export_occupied(bxg_pmap m_, float* out_xyz, size_t cap, size_t* n_out, doub
   }
   BXG_CUDA(m, m->s_tmp.ensure(8));
   BXG_CUDA(m, cudaMemsetAsync(m->s_tmp.p, 0, 8, m->stream));
-  const size_t threads = size_t(n_leaves) * m->dm.lwords;
   const size_t wcap = dout ? cap : 0;
-  if (threads) {
-    k_export_occupied<<<unsigned((threads + 255) / 256), 256, 0, m->stream>>>(
+  if (n_leaves) {
+    k_export_occupied<<<(n_leaves + 8 * kExportLeaves - 1) / (8 * kExportLeaves), 256, 0,
+                        m->stream>>>(
         m->dm, n_leaves, static_cast<float*>(dout), wcap, m->s_tmp.as<unsigned long long>(),
         m_->opt.occupancy_threshold_log, m->res, min_z, max_z);
     BXG_LAUNCHED(m);
