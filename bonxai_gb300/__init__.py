@@ -377,10 +377,13 @@ class VoxelGrid(_Handle):
         st = self.lib.bxg_grid_serialize(self.h, type_name.encode(), None, 0, C.byref(n))
         if st not in (0, 7):
             self._check(st)
-        buf = C.create_string_buffer(n.value)
-        self._check(self.lib.bxg_grid_serialize(self.h, type_name.encode(), buf, n.value,
+        # a bytes object of that size, filled before anyone else sees it
+        new = C.pythonapi.PyBytes_FromStringAndSize
+        new.restype, new.argtypes = C.py_object, [C.c_char_p, C.c_ssize_t]
+        out = new(None, n.value)
+        self._check(self.lib.bxg_grid_serialize(self.h, type_name.encode(), out, n.value,
                                                 C.byref(n)))
-        return buf.raw[:n.value]
+        return out
 
     def deserialize(self, data: bytes):
         self._check(self.lib.bxg_grid_deserialize(self.h, data, len(data)))

@@ -358,24 +358,6 @@ uint8_t* pre_bytes(MapCore* m, uint32_t cap, bool with_min) {
   return with_min ? m->s_dedup2.as<uint8_t>() + size_t(cap) * 4 : m->s_dedup2.as<uint8_t>();
 }
 
-// Runs a batch that creates topology, retrying once pools have grown.
-template <class F>
-int run_with_growth(MapCore* m, F&& body) {
-  for (int attempt = 0; attempt < 12; attempt++) {
-    int st = body();
-    if (st) return st;
-    uint32_t err = 0;
-    st = core_sync(m, &err);
-    if (st == BXG_OK) return core_maintain(m);
-    if (!(err & (ERR_POOL_INNER | ERR_POOL_LEAF | ERR_HASH_FULL)) ||
-        (err & (ERR_WAIT | ERR_RAY_TOO_LONG | ERR_SCRATCH)))
-      return st;
-    const int g = core_grow_for(m, err);
-    if (g) return g;
-  }
-  return set_error(m, BXG_ERR_OUT_OF_POOL, "pools could not grow enough");
-}
-
 int grid_set_values_dev(bxg_grid g, const int32_t* dxyz, const void* dvals, uint32_t n,
                         uint8_t* was_on) {
   MapCore* m = &g->core;

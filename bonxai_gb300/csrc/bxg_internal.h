@@ -160,6 +160,24 @@ inline unsigned long long* stats_of(const MapCore* m) {
 void launch_dedup_clear(MapCore* m, uint4* tab, uint32_t cap);
 // Inserts the non-empty buckets of old_b[0..old_cap) into the table of M.
 void launch_rehash(MapCore* m, const uint4* old_b, uint32_t old_cap, const DMap& M);
+// Runs a batch that creates topology, retrying once pools have grown.
+template <class F>
+int run_with_growth(MapCore* m, F&& body) {
+  for (int attempt = 0; attempt < 12; attempt++) {
+    int st = body();
+    if (st) return st;
+    uint32_t err = 0;
+    st = core_sync(m, &err);
+    if (st == BXG_OK) return core_maintain(m);
+    if (!(err & (ERR_POOL_INNER | ERR_POOL_LEAF | ERR_HASH_FULL)) ||
+        (err & (ERR_WAIT | ERR_RAY_TOO_LONG | ERR_SCRATCH)))
+      return st;
+    const int g = core_grow_for(m, err);
+    if (g) return g;
+  }
+  return set_error(m, BXG_ERR_OUT_OF_POOL, "pools could not grow enough");
+}
+
 // Text of the last failed create call on this host thread.
 void set_create_error(const std::string& msg);
 const MapCore* core_of_handle(const void* handle);
