@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(kMarkThreads, kMarkBlocksPerSM) k_tick_mark(
       const uint32_t a = uint32_t(lo - pre[s]), b = uint32_t(stop - pre[s]);
       uint32_t visited = 0;
       mark_scan(T.M, Q, A.cast + T.pt_begin, min(a, n), min(b, n), max(a, n) - n, max(b, n) - n,
-                kMarkThreads, T.ox, T.oy, T.oz, S, visited);
+                kMarkThreads, kMarkThreads, T.ox, T.oy, T.oz, S, visited);
       visited = __reduce_add_sync(0xffffffffu, visited);
       if ((threadIdx.x & 31) == 0 && visited)
         atomicAdd(reinterpret_cast<unsigned long long*>(T.M.ctr + C_STATS) + S_VISITED,
@@ -345,7 +345,7 @@ __global__ void __launch_bounds__(256, 8) k_tick_apply(const TickArgs* __restric
     const TickScan& T = sc[s];
     const uint32_t SR = T.Q.SR;
     const uint32_t rz = i / (SR * SR), ry = (i - rz * SR * SR) / SR, rx = i - (rz * SR + ry) * SR;
-    apply_row(T.M, T.Q, rx, 4u * ry + (t & 3u), 4u * rz + ((t >> 2) & 3u), T.u, T.o.miss, T.o.cmin,
+    apply_row<1>(T.M, T.Q, rx, 4u * ry + (t & 3u), 4u * rz + ((t >> 2) & 3u), T.u, T.o.miss, T.o.cmin,
               W.rows[threadIdx.x >> 5], updated);
   }
   if (cur != kNone) count();

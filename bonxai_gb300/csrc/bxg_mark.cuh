@@ -96,9 +96,10 @@ __device__ __forceinline__ uint32_t apply_leaf_slot(const DMap& M, int lx, int l
 // depth frame) the ORs that meet in few words of L2. Kernel times on a GB300,
 // L2 warm, against tasks of rays whose segments were found by a prefix and a
 // search and walked with integer divisions (the form before): LiDAR 131k points,
-// 9.3 M cells, 28 us (62); depth 307k points, 10.5 M cells, 62 us (105); room
-// 60k points 20 us (30). Of that, without the far ORs: 26, 39 and 19 us; with
-// every lane's cells ORed, neighbours' too: 36, 65 and 21 us. Measured and not
+// 9.3 M cells, 25 us (62); depth 307k points, 10.5 M cells, 59 us (105); room
+// 60k points 18 us (30); 2k points 9.5 us (16). Before the near cells got blocks of their
+// own these were 28, 62, 20 and 14 us, of which without the far ORs 26, 39, 19
+// and 13 us, and with every lane's cells ORed, neighbours' too, 36, 65, 21 us. Measured and not
 // kept: rays sorted by direction and collected per block in shared memory, in
 // a dense box of leaves (LiDAR 55 us, depth 60 us: scanning the box costs more
 // than the ORs it saves), in a hash of leaves or behind a table (80-100 us: a
@@ -281,14 +282,14 @@ struct MarkShared {
   uint32_t roots[kRootFlagWords];
 };
 
-// A block's part of a scan's rays: the near cells of rays r, r + step, ... < r_end (r: the
-// first thread's), and the segments s, s + step, ... < s_end likewise (step a multiple of
+// A block's part of a scan's rays: the near cells of rays r, r + r_step, ... < r_end (r: the
+// first thread's), and the segments s, s + s_step, ... < s_end likewise (steps a multiple of
 // kMarkThreads). All threads of a block of kMarkThreads. Adds the cells walked to `visited`.
 __device__ __forceinline__ void mark_scan(const DMap& M, const ScanCube& Q,
                                           const int4* __restrict__ cast, uint32_t r,
                                           uint32_t r_end, uint32_t s, uint32_t s_end,
-                                          uint32_t step, int ox, int oy, int oz, MarkShared& S,
-                                          uint32_t& visited) {
+                                          uint32_t r_step, uint32_t s_step, int ox, int oy, int oz,
+                                          MarkShared& S, uint32_t& visited) {
   const int qx = ox - Q.x0, qy = oy - Q.y0, qz = oz - Q.z0;  // the origin in the cube
   // the neighbourhood's lowest cell, from the origin
   const int wx = ((qx >> 3) - kNearNB) * 8 - qx, wy = ((qy >> 3) - kNearNB) * 8 - qy,
@@ -298,7 +299,7 @@ __device__ __forceinline__ void mark_scan(const DMap& M, const ScanCube& Q,
     for (uint32_t t = threadIdx.x; t < kNearWords; t += kMarkThreads) S.near[t] = 0u;
   for (uint32_t t = threadIdx.x; t < root_words; t += kMarkThreads) S.roots[t] = 0u;
   __syncthreads();
-  for (uint32_t i = r + threadIdx.x; i < r_end; i += step) {
+  for (uint32_t i = r + threadIdx.x; i < r_end; i += r_step) {
     const MarkRay q = mark_ray(M, Q, cast[i], ox, oy, oz);
     if (!q.m) continue;
     visited += q.m;
@@ -318,7 +319,7 @@ __device__ __forceinline__ void mark_scan(const DMap& M, const ScanCube& Q,
       flag_roots(Q, qx + ax, qy + ay, qz + az, qx + bx, qy + by, qz + bz, S.roots);
     }
   }
-  for (uint32_t i0 = s + (threadIdx.x & ~31u); i0 < s_end; i0 += step) {
+  for (uint32_t i0 = s + (threadIdx.x & ~31u); i0 < s_end; i0 += s_step) {
     const uint32_t i = i0 + (threadIdx.x & 31);
     const uint32_t seg = i < s_end ? Q.segs[i] : 0u;
     const MarkRay q = mark_ray(M, Q, cast[seg >> 8], ox, oy, oz);
@@ -372,7 +373,10 @@ __device__ __forceinline__ void mark_scan(const DMap& M, const ScanCube& Q,
 // cells in 18 k leaves: 24 us (37 with eight lanes for each leaf of a list, a
 // lane 64 cells and two rounds of eight loads); 8 maps of few points, 225 k leaves
 // with 29 cells each: 82 us (107 with the whole warp on one leaf's 64 rows at a
-// time: most rows have no marked cell).
+// time: most rows have no marked cell). One scan cannot fill the chip and loads two rows
+// at a time, at four blocks per SM (2k points 12.1 us against 13.8, room 11.9 against
+// 13.4); a tick can, and takes one at eight blocks per SM (64 maps: 1.28 ms; two at
+// a time 1.34).
 // ---------------------------------------------------------------------------
 constexpr int kApplyWarps = 8;
 struct ApplyShared {
@@ -399,7 +403,9 @@ __device__ __forceinline__ uint32_t miss_run(int4& v, uint32_t nib, int32_t u, i
   return fresh;
 }
 
-// Blocks 4 rx .. 4 rx + 3 of the row (by, bz), in leaves of the cube.
+// Blocks 4 rx .. 4 rx + 3 of the row (by, bz), in leaves of the cube. ROWS: listed rows
+// that a lane loads before it updates them.
+template <int ROWS>
 __device__ __forceinline__ void apply_row(const DMap& M, const ScanCube& Q, uint32_t rx,
                                           uint32_t by, uint32_t bz, int32_t u, int32_t miss,
                                           int32_t cmin, uint2* list, uint32_t& updated) {
@@ -441,26 +447,35 @@ __device__ __forceinline__ void apply_row(const DMap& M, const ScanCube& Q, uint
     }
   }
   __syncwarp();
-  for (uint32_t i = lane; i < total; i += 32) {
-    const uint2 e = list[i];
-    const unsigned long long row = (static_cast<unsigned long long>(e.y) << 24) | (e.x >> 8);
-    const uint32_t cells = e.x & 0xFFu;
-    int4* c = reinterpret_cast<int4*>(M.ldata) + 2 * row;
-    int4 v[2];
-    if (cells & 0xFu) v[0] = c[0];
-    if (cells & 0xF0u) v[1] = c[1];
-    uint32_t fresh = 0;
+  for (uint32_t i = lane; i < total; i += 32 * ROWS) {
+    uint2 e[ROWS];
+    int4 v[ROWS][2];
+    auto row_of = [](uint2 x) { return (static_cast<unsigned long long>(x.y) << 24) | (x.x >> 8); };
 #pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const uint32_t nib = (cells >> (4 * q)) & 0xFu;
-      if (!nib) continue;
-      bool changed = false;
-      fresh |= miss_run(v[q], nib, u, miss, cmin, changed, updated) << (4 * q);
-      if (changed) c[q] = v[q];
+    for (int p = 0; p < ROWS; ++p) {
+      e[p] = i + 32 * p < total ? list[i + 32 * p] : make_uint2(0u, 0u);
+      const int4* c = reinterpret_cast<const int4*>(M.ldata) + 2 * row_of(e[p]);
+      if (e[p].x & 0xFu) v[p][0] = c[0];
+      if (e[p].x & 0xF0u) v[p][1] = c[1];
     }
-    // the row's mask byte, in its 32-bit word
-    if (fresh)
-      red_or(reinterpret_cast<uint32_t*>(M.lmask) + (row >> 2), fresh << (8u * (row & 3u)));
+#pragma unroll
+    for (int p = 0; p < ROWS; ++p) {
+      const unsigned long long row = row_of(e[p]);
+      const uint32_t cells = e[p].x & 0xFFu;
+      int4* c = reinterpret_cast<int4*>(M.ldata) + 2 * row;
+      uint32_t fresh = 0;
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const uint32_t nib = (cells >> (4 * q)) & 0xFu;
+        if (!nib) continue;
+        bool changed = false;
+        fresh |= miss_run(v[p][q], nib, u, miss, cmin, changed, updated) << (4 * q);
+        if (changed) c[q] = v[p][q];
+      }
+      // the row's mask byte, in its 32-bit word
+      if (fresh)
+        red_or(reinterpret_cast<uint32_t*>(M.lmask) + (row >> 2), fresh << (8u * (row & 3u)));
+    }
   }
   __syncwarp();
 }
@@ -520,7 +535,7 @@ __device__ __forceinline__ void apply_scan(const DMap& M, const ScanCube& Q, uin
         0xffffffffu, ((v >> lane) & 1u) && uint32_t(__popc(v & ((1u << lane) - 1u))) == k - pre[lo])) - 1);
     const uint32_t rz = i / (Q.SR * Q.SR), ry = (i - rz * Q.SR * Q.SR) / Q.SR,
                    rx = i - (rz * Q.SR + ry) * Q.SR;
-    apply_row(M, Q, rx, 4u * ry + (t & 3u), 4u * rz + ((t >> 2) & 3u), u, miss, cmin, list,
+    apply_row<2>(M, Q, rx, 4u * ry + (t & 3u), 4u * rz + ((t >> 2) & 3u), u, miss, cmin, list,
               updated);
   }
 }
