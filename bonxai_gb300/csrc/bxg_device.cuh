@@ -200,26 +200,43 @@ __device__ __forceinline__ uint32_t cell_hash(int x, int y, int z) {
 // ---------------------------------------------------------------------------
 // slot allocation
 // ---------------------------------------------------------------------------
+// A counter step for each of the threads that are here together, as one atomic per warp:
+// thousands of new nodes take their slots from one word, and its atomics with a
+// result come out of L2 one after the other.
+__device__ __forceinline__ uint32_t counter_step(uint32_t* c) {
+  const unsigned here = __activemask();
+  const unsigned lane = threadIdx.x & 31;
+  const int lead = __ffs(static_cast<int>(here)) - 1;
+  uint32_t base = 0;
+  if (static_cast<int>(lane) == lead) base = atomicAdd(c, static_cast<uint32_t>(__popc(here)));
+  return __shfl_sync(here, base, lead) + __popc(here & ((1u << lane) - 1u));
+}
+// Sets an error bit that many threads may set.
+__device__ __forceinline__ void set_err_once(const DMap& M, uint32_t bit) {
+  if (!(ld_volatile(M.ctr + C_ERR) & bit)) set_err(M, bit);
+}
 __device__ __forceinline__ uint32_t alloc_inner(const DMap& M) {
-  const uint32_t i = atomicAdd(M.ctr + C_INNER, 1u);
+  const uint32_t i = counter_step(M.ctr + C_INNER);
   if (i >= M.icap) {
-    set_err(M, ERR_POOL_INNER);
+    set_err_once(M, ERR_POOL_INNER);
     return kNone;
   }
   return i;
 }
 // Released leaves are reused first (their masks and cells are all zero). The
 // free stack is only filled by releaseUnusedMemory, so kernels launched while
-// the host knows it is empty skip the probe.
-__device__ __forceinline__ uint32_t alloc_leaf(const DMap& M) {
+// the host knows it is empty skip the probe. A pool that was found full stays
+// so for the launch: later requests fail without touching its counter.
+__device__ __forceinline__ uint32_t alloc_leaf(const DMap& M, uint32_t err) {
   if (M.has_free && ld_volatile(M.ctr + C_FREE_LEAF) > 0) {
     const int prev = static_cast<int>(atomicSub(M.ctr + C_FREE_LEAF, 1u));
     if (prev > 0) return M.lfree[prev - 1];
     atomicAdd(M.ctr + C_FREE_LEAF, 1u);  // lost the race for the last entry
   }
-  const uint32_t i = atomicAdd(M.ctr + C_LEAF, 1u);
+  if (err & ERR_POOL_LEAF) return kNone;
+  const uint32_t i = counter_step(M.ctr + C_LEAF);
   if (i >= M.lcap) {
-    set_err(M, ERR_POOL_LEAF);
+    set_err_once(M, ERR_POOL_LEAF);
     return kNone;
   }
   return i;
@@ -282,7 +299,7 @@ static __device__ __noinline__ uint32_t root_get_or_create(const DMap& M, int x,
       if (eq4(v, kEmpty)) {
         const uint32_t in = alloc_inner(M);
         st_publish(&b->w, in);
-        atomicAdd(M.ctr + C_ROOTS, 1u);
+        counter_step(M.ctr + C_ROOTS);
         return in;
       }
       if (!key_eq(v, x, y, z)) continue;
@@ -322,9 +339,10 @@ static __device__ __noinline__ uint32_t leaf_get_or_create(const DMap& M, uint32
   for (int it = 0; it < kSpinLimit; ++it) {
     if (c < kPending) return c;
     if (c == kNone) {
+      const uint32_t err = ld_volatile(M.ctr + C_ERR);  // on its way while the CAS is
       const uint32_t old = atomicCAS(slot, kNone, kPending);
       if (old == kNone) {
-        const uint32_t lf = alloc_leaf(M);
+        const uint32_t lf = alloc_leaf(M, err);
         st_publish(slot, lf);
         if (lf != kNone) {  // read only by later kernels (iteration, release)
           M.lkey[lf] = make_int4(lx, ly, lz, static_cast<int>(in));
