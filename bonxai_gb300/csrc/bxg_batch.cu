@@ -437,7 +437,7 @@ __global__ void __launch_bounds__(256, U == 2 ? 3 : 4) k_tick(const TickArgs* __
       valid = e.w != EP_SKIP;
       if (valid && dedup_lookup(A.tab + S.tab_begin, S.tmask, e.x, e.y, e.z) ==
                        static_cast<uint32_t>(i - S.pt_begin))
-        add = winner_apply(S.M, e, S.u, S.o);
+        add = winner_apply(S.M, e, kPending, S.u, S.o);
     }
     const uint32_t s0 = __shfl_sync(0xffffffffu, s, 0);
     const bool uniform = __all_sync(0xffffffffu, !in || s == s0);
@@ -599,12 +599,6 @@ int bfail(bxg_batch b, int st, const std::string& m) {
     }                                                                                  \
   } while (0)
 
-uint32_t pow2_at_least(uint64_t v) {
-  uint32_t p = 64;
-  while (p < v) p <<= 1;
-  return p;
-}
-
 template <int W, int U>
 int occupancy_grid(bxg_batch b, size_t smem) {
   int per_sm = 0;
@@ -760,7 +754,7 @@ int bxg_batch_insert_f32(bxg_batch b, const bxg_pmap* maps, size_t n_scans, cons
 
   // Device buffers (growing them invalidates the captured graph).
   uint64_t tab_total = 0;
-  for (size_t s = 0; s < n_scans; s++) tab_total += pow2_at_least(2 * (offsets[s + 1] - offsets[s]));
+  for (size_t s = 0; s < n_scans; s++) tab_total += dedup_entries(offsets[s + 1] - offsets[s]);
   const void* dpts = xyz;
   const int pts_dev = ptr_device(xyz);
   // points in another GPU's memory are copied like host points (never read in place)
@@ -827,7 +821,7 @@ int bxg_batch_insert_f32(bxg_batch b, const bxg_pmap* maps, size_t n_scans, cons
                pm->opt.clamp_max_log};
     S.pt_begin = offsets[s];
     S.n = uint32_t(offsets[s + 1] - offsets[s]);
-    const uint32_t tcap = pow2_at_least(2 * uint64_t(S.n));
+    const uint32_t tcap = dedup_entries(S.n);
     S.tab_begin = tb;
     S.tmask = tcap - 1;
     tb += tcap;

@@ -560,7 +560,10 @@ __device__ __forceinline__ void winners_block(const DMap& M, const int4* __restr
   if (i < n) {
     e = ep[i];
     if (e.w == EP_HIT || e.w == EP_MISS) {
-      if (dedup_lookup(tab, tmask, e.x, e.y, e.z) == i) add = winner_apply(M, e, u, o);
+      // the root's bucket is on its way while the table's is
+      const int32_t rm = root_mask(M);
+      const uint32_t in = root_probe_fast(M, e.x & rm, e.y & rm, e.z & rm);
+      if (dedup_lookup(tab, tmask, e.x, e.y, e.z) == i) add = winner_apply(M, e, in, u, o);
     }
   }
   const unsigned lane = threadIdx.x & 31, wid = threadIdx.x >> 5;

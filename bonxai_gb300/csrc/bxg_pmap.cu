@@ -315,12 +315,6 @@ using namespace bxg;
 
 namespace {
 
-uint32_t next_pow2(uint64_t v) {
-  uint32_t p = 64;
-  while (p < v) p <<= 1;
-  return p;
-}
-
 Opts opts_of(const bxg_pmap_s* pm) {
   return Opts{pm->opt.prob_miss_log, pm->opt.prob_hit_log, pm->opt.clamp_min_log,
               pm->opt.clamp_max_log};
@@ -346,7 +340,7 @@ template <class Launch>
 int endpoint_phase(bxg_pmap_s* pm, uint32_t n, int ox, int oy, int oz, const ScanCube& cube,
                    Launch&& launch_ep) {
   MapCore* m = &pm->core;
-  const uint32_t tcap = next_pow2(uint64_t(n) * 2);
+  const uint32_t tcap = dedup_entries(n);
   BXG_CUDA(m, m->s_ep.ensure(size_t(n) * 16));
   const void* old_tab = m->s_dedup.p;
   BXG_CUDA(m, m->s_dedup.ensure(size_t(tcap) * 16));

@@ -217,10 +217,20 @@ __device__ __forceinline__ uint32_t chebyshev(int ox, int oy, int oz, int x, int
 // (probabilistic_map.cpp:35-41,49-54) and its ray is cast (returns true). The
 // winner owns its cell -- no other thread writes it in this phase -- so the
 // word it reads is the pre-scan word. If the pool is full the ray is still
-// listed and the endpoint is completed after the pool grows.
-__device__ __forceinline__ bool winner_apply(const DMap& M, int4 e, int32_t u, const Opts& o) {
-  const uint32_t lf = leaf_of(M, e.x, e.y, e.z, true);
-  if (lf == kNone) return true;
+// listed and the endpoint is completed after the pool grows. in: what
+// root_probe_fast said of the cell's root.
+__device__ __forceinline__ bool winner_apply(const DMap& M, int4 e, uint32_t in, int32_t u,
+                                             const Opts& o) {
+  const int32_t rm = root_mask(M);
+  if (in == kPending) in = root_get_or_create(M, e.x & rm, e.y & rm, e.z & rm);
+  if (in == kNone) return true;
+  const uint32_t ii = inner_index(M, e.x, e.y, e.z);
+  uint32_t lf = M.ichild[static_cast<size_t>(in) * M.isize + ii];
+  if (lf >= kPending) {
+    const int32_t lm = leaf_mask(M);
+    lf = leaf_get_or_create(M, in, ii, e.x & lm, e.y & lm, e.z & lm);
+    if (lf == kNone) return true;
+  }
   const uint32_t ci = leaf_index(M, e.x, e.y, e.z);
   int32_t* cp = reinterpret_cast<int32_t*>(M.ldata) + size_t(lf) * M.lsize + ci;
   const bool on = cell_is_on(M, lf, ci);
