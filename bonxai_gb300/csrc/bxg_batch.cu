@@ -668,66 +668,13 @@ cudaError_t enqueue_tick(bxg_batch b, size_t param_bytes, size_t smem, bool mark
 
 }  // namespace
 
-extern "C" {
-
-int bxg_batch_create(bxg_batch* out, const bxg_config* cfg_in) {
-  if (!out) return BXG_ERR_INVALID_ARG;
-  *out = nullptr;
-  bxg_config cfg;
-  bxg_config_default(&cfg);
-  if (cfg_in) cfg = *cfg_in;
-  int ndev = 0;
-  if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) {
-    cudaGetLastError();
-    return BXG_ERR_NO_DEVICE;
-  }
-  bxg_batch b = new bxg_batch_s();
-  if (cfg.device >= 0) cudaSetDevice(cfg.device);
-  cudaGetDevice(&b->device);
-  cudaDeviceGetAttribute(&b->sm_count, cudaDevAttrMultiProcessorCount, b->device);
-  b->rays_per_warp = cfg.rays_per_warp == 2 || cfg.rays_per_warp == 4 ? cfg.rays_per_warp : 1;
-  b->ray_unroll = cfg.ray_unroll == 2 ? 2 : 1;
-  b->use_graph = (cfg.flags & 4u) == 0;  // BXG_FLAG_NO_GRAPH
-  if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaEventCreate(&b->ev0) != cudaSuccess || cudaEventCreate(&b->ev1) != cudaSuccess) {
-    cudaGetLastError();
-    delete b;
-    return BXG_ERR_CUDA;
-  }
-  const int smem = int(tick_smem(kMaxTickScans));
-  cudaFuncSetAttribute(k_tick<32, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  cudaFuncSetAttribute(k_tick<16, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  cudaFuncSetAttribute(k_tick<8, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  cudaFuncSetAttribute(k_tick<32, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  cudaFuncSetAttribute(k_tick<16, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  cudaFuncSetAttribute(k_tick<8, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  b->grid_mark = b->sm_count * kMarkBlocksPerSM;
-  cudaGetLastError();
-  const size_t pbytes = 256 + kMaxTickScans * sizeof(TickScan);
-  if (cudaMallocHost(reinterpret_cast<void**>(&b->h_args), pbytes) != cudaSuccess ||
-      b->params.ensure(pbytes) != cudaSuccess) {
-    cudaGetLastError();
-    delete b;
-    return BXG_ERR_CUDA;
-  }
-  b->h_scans = reinterpret_cast<TickScan*>(reinterpret_cast<uint8_t*>(b->h_args) + 256);
-  *out = b;
-  return BXG_OK;
-}
-
-int bxg_batch_destroy(bxg_batch b) {
-  delete b;
-  return BXG_OK;
-}
-
-const char* bxg_batch_last_error(bxg_batch b) { return b ? b->err.c_str() : "null handle"; }
-
-int bxg_batch_insert_f32(bxg_batch b, const bxg_pmap* maps, size_t n_scans, const float* xyz,
-                         const uint64_t* offsets, const float* origins, const double* max_ranges,
-                         uint64_t* ray_cells) {
+namespace bxg {
+int batch_insert(bxg_batch b, const bxg_pmap* maps, size_t n_scans, const float* xyz,
+                 const float* const* parts, const uint64_t* offsets, const float* origins,
+                 const double* max_ranges, uint64_t* ray_cells) {
   if (!b) return BXG_ERR_INVALID_ARG;
   if (!n_scans) return BXG_OK;
-  if (!maps || !xyz || !offsets || !origins || !max_ranges)
+  if (!maps || !offsets || !origins || !max_ranges)
     return bfail(b, BXG_ERR_INVALID_ARG, "null argument");
   if (n_scans > kMaxTickScans)
     return bfail(b, BXG_ERR_INVALID_ARG, "at most 128 scans per tick");
@@ -756,7 +703,7 @@ int bxg_batch_insert_f32(bxg_batch b, const bxg_pmap* maps, size_t n_scans, cons
   uint64_t tab_total = 0;
   for (size_t s = 0; s < n_scans; s++) tab_total += dedup_entries(offsets[s + 1] - offsets[s]);
   const void* dpts = xyz;
-  const int pts_dev = ptr_device(xyz);
+  const int pts_dev = parts ? kPtrHost : ptr_device(xyz);
   // points in another GPU's memory are copied like host points (never read in place)
   const bool host_pts = pts_dev != b->device && pts_dev != kPtrManaged;
   bool realloc = false;
@@ -774,7 +721,13 @@ int bxg_batch_insert_f32(bxg_batch b, const bxg_pmap* maps, size_t n_scans, cons
     BB_CUDA(b, cudaMallocHost(reinterpret_cast<void**>(&b->h_back), kBackBytes));
   }
   if (host_pts) {
-    if (pts_dev >= 0)
+    if (parts) {
+      for (size_t s = 0; s < n_scans; s++)
+        if (offsets[s + 1] > offsets[s])
+          BB_CUDA(b, cudaMemcpyAsync(b->pts.as<float>() + 3 * offsets[s], parts[s],
+                                     (offsets[s + 1] - offsets[s]) * 12, cudaMemcpyHostToDevice,
+                                     b->stream));
+    } else if (pts_dev >= 0)
       BB_CUDA(b, cudaMemcpyPeerAsync(b->pts.p, b->device, xyz, pts_dev, total * 12, b->stream));
     else
       BB_CUDA(b, cudaMemcpyAsync(b->pts.p, xyz, total * 12, cudaMemcpyHostToDevice, b->stream));
@@ -974,7 +927,70 @@ int bxg_batch_insert_f32(bxg_batch b, const bxg_pmap* maps, size_t n_scans, cons
   }
   return status;
 }
+}  // namespace bxg
 
+extern "C" {
+
+int bxg_batch_create(bxg_batch* out, const bxg_config* cfg_in) {
+  if (!out) return BXG_ERR_INVALID_ARG;
+  *out = nullptr;
+  bxg_config cfg;
+  bxg_config_default(&cfg);
+  if (cfg_in) cfg = *cfg_in;
+  int ndev = 0;
+  if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) {
+    cudaGetLastError();
+    return BXG_ERR_NO_DEVICE;
+  }
+  bxg_batch b = new bxg_batch_s();
+  if (cfg.device >= 0) cudaSetDevice(cfg.device);
+  cudaGetDevice(&b->device);
+  cudaDeviceGetAttribute(&b->sm_count, cudaDevAttrMultiProcessorCount, b->device);
+  b->rays_per_warp = cfg.rays_per_warp == 2 || cfg.rays_per_warp == 4 ? cfg.rays_per_warp : 1;
+  b->ray_unroll = cfg.ray_unroll == 2 ? 2 : 1;
+  b->use_graph = (cfg.flags & 4u) == 0;  // BXG_FLAG_NO_GRAPH
+  if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaEventCreate(&b->ev0) != cudaSuccess || cudaEventCreate(&b->ev1) != cudaSuccess) {
+    cudaGetLastError();
+    delete b;
+    return BXG_ERR_CUDA;
+  }
+  const int smem = int(tick_smem(kMaxTickScans));
+  cudaFuncSetAttribute(k_tick<32, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  cudaFuncSetAttribute(k_tick<16, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  cudaFuncSetAttribute(k_tick<8, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  cudaFuncSetAttribute(k_tick<32, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  cudaFuncSetAttribute(k_tick<16, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  cudaFuncSetAttribute(k_tick<8, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  b->grid_mark = b->sm_count * kMarkBlocksPerSM;
+  cudaGetLastError();
+  const size_t pbytes = 256 + kMaxTickScans * sizeof(TickScan);
+  if (cudaMallocHost(reinterpret_cast<void**>(&b->h_args), pbytes) != cudaSuccess ||
+      b->params.ensure(pbytes) != cudaSuccess) {
+    cudaGetLastError();
+    delete b;
+    return BXG_ERR_CUDA;
+  }
+  b->h_scans = reinterpret_cast<TickScan*>(reinterpret_cast<uint8_t*>(b->h_args) + 256);
+  *out = b;
+  return BXG_OK;
+}
+
+int bxg_batch_destroy(bxg_batch b) {
+  delete b;
+  return BXG_OK;
+}
+
+const char* bxg_batch_last_error(bxg_batch b) { return b ? b->err.c_str() : "null handle"; }
+
+int bxg_batch_insert_f32(bxg_batch b, const bxg_pmap* maps, size_t n_scans, const float* xyz,
+                         const uint64_t* offsets, const float* origins, const double* max_ranges,
+                         uint64_t* ray_cells) {
+  if (!b) return BXG_ERR_INVALID_ARG;
+  if (!n_scans) return BXG_OK;
+  if (!xyz) return bfail(b, BXG_ERR_INVALID_ARG, "null argument");
+  return batch_insert(b, maps, n_scans, xyz, nullptr, offsets, origins, max_ranges, ray_cells);
+}
 int bxg_batch_phase_ms(bxg_batch b, double out[6]) {
   if (!b || !out) return BXG_ERR_INVALID_ARG;
   for (int k = 0; k < 6; k++) out[k] = b->phase_ms[k];

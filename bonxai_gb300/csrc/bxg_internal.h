@@ -248,6 +248,11 @@ int leaf_dir_for_scan(bxg_pmap_s* pm, int ox, int oy, int oz, LeafDir* D, size_t
 // idempotent endpoint completion and ray phases on the map's own stream.
 int pmap_complete_scan(bxg_pmap_s* pm, const int4* d_cast, const uint32_t* d_count,
                        uint32_t cap, int ox, int oy, int oz, int32_t u);
+// bxg_batch_insert_f32, with the points of scan s either at xyz + 3 offsets[s] or, with
+// parts, in host memory at parts[s].
+int batch_insert(bxg_batch b, const bxg_pmap* maps, size_t n_scans, const float* xyz,
+                 const float* const* parts, const uint64_t* offsets, const float* origins,
+                 const double* max_ranges, uint64_t* ray_cells);
 // Grows the map's pools so that the next scan has at least `leaves` free leaf
 // slots and the root hash stays under its load factor.
 int core_reserve(MapCore* m, size_t leaves, size_t inners);

@@ -24,6 +24,7 @@
 #include <algorithm>
 #include <chrono>
 #include <condition_variable>
+#include <cstdlib>
 #include <cstring>
 #include <deque>
 #include <mutex>
@@ -82,6 +83,115 @@ using namespace bxg;
 using Clock = std::chrono::steady_clock;
 
 namespace {
+// Page-locked host buffers of the requests' inputs, kept between requests: the client's
+// copy into one touches no new pages, and the worker's copy to the GPU reads it in place.
+// A client only takes a free buffer, else plain memory (page-locking is a call into the
+// driver that may not be made during a stream capture); the worker makes the buffers that were
+// missed, until kMost bytes are held. They are freed with the server.
+class HostPool {
+ public:
+  static constexpr size_t kMost = size_t(256) << 20;
+  static constexpr size_t kLeast = size_t(64) << 10;
+  // *cap: the size of a pooled buffer, 0 for plain memory.
+  void* take(size_t bytes, size_t* cap) {
+    size_t c = 0;
+    const int k = class_of(bytes, &c);
+    if (k < kClasses) {
+      std::lock_guard<std::mutex> lk(mu_);
+      if (!free_[k].empty()) {
+        void* p = free_[k].back();
+        free_[k].pop_back();
+        *cap = c;
+        return p;
+      }
+      missed_[k]++;
+    }
+    *cap = 0;
+    return std::malloc(bytes ? bytes : 1);
+  }
+  void give(void* p, size_t cap) {
+    if (!cap) {
+      std::free(p);
+      return;
+    }
+    size_t c = 0;
+    const int k = class_of(cap, &c);
+    std::lock_guard<std::mutex> lk(mu_);
+    free_[k].push_back(p);
+  }
+  // (worker) Makes a buffer for each request that found none.
+  void refill() {
+    for (int k = 0; k < kClasses; ++k) {
+      const size_t c = kLeast << k;
+      for (;;) {
+        {
+          std::lock_guard<std::mutex> lk(mu_);
+          if (!missed_[k] || held_ + c > kMost) {
+            missed_[k] = 0;
+            break;
+          }
+          missed_[k]--;
+          held_ += c;
+        }
+        void* p = nullptr;
+        if (cudaMallocHost(&p, c) != cudaSuccess) {
+          cudaGetLastError();
+          return;
+        }
+        std::lock_guard<std::mutex> lk(mu_);
+        free_[k].push_back(p);
+      }
+    }
+  }
+  ~HostPool() {
+    for (auto& f : free_)
+      for (void* p : f) cudaFreeHost(p);
+  }
+
+ private:
+  static constexpr int kClasses = 13;  // 64 KB .. 256 MB
+  static int class_of(size_t bytes, size_t* c) {
+    int k = 0;
+    for (*c = kLeast; *c < bytes; *c <<= 1) ++k;
+    return k;
+  }
+  std::mutex mu_;
+  std::vector<void*> free_[kClasses];
+  size_t missed_[kClasses] = {0};
+  size_t held_ = 0;
+};
+
+// An input array in a buffer of the pool.
+template <class T>
+class HostArray {
+ public:
+  HostArray() = default;
+  HostArray(const HostArray&) = delete;
+  HostArray& operator=(const HostArray&) = delete;
+  ~HostArray() { reset(); }
+  bool assign(HostPool* pool, const T* src, size_t n) {
+    reset();
+    p_ = static_cast<T*>(pool->take(n * sizeof(T), &cap_));
+    if (!p_) return false;
+    pool_ = pool;
+    n_ = n;
+    if (n) std::memcpy(p_, src, n * sizeof(T));
+    return true;
+  }
+  void reset() {
+    if (p_) pool_->give(p_, cap_);
+    p_ = nullptr;
+    n_ = 0;
+  }
+  const T* data() const { return p_; }
+  size_t size() const { return n_; }
+
+ private:
+  HostPool* pool_ = nullptr;
+  T* p_ = nullptr;
+  size_t n_ = 0, cap_ = 0;
+};
+
 enum Kind : int { K_INSERT = 0, K_QUERY = 1, K_OCCUPIED = 2, K_CLEAR = 3 };
 
 struct Request {
@@ -89,10 +199,10 @@ struct Request {
   Kind kind = K_INSERT;
   uint32_t map = 0;
   bool discard = false;
-  std::vector<float> pts;
+  HostArray<float> pts;
   float origin[3] = {0, 0, 0};
   double max_range = 0;
-  std::vector<int32_t> coords;
+  HostArray<int32_t> coords;
   int mode = 0;
   // results
   bool done = false;
@@ -107,6 +217,7 @@ struct Request {
 }  // namespace
 
 struct bxg_server_s {
+  HostPool pool;  // outlives the requests, which the destructor below deletes
   int device = 0;
   std::vector<bxg_pmap> maps;
   bxg_batch batch = nullptr;
@@ -128,9 +239,6 @@ struct bxg_server_s {
   std::thread worker;
   // staging
   DevBuf d_pts, d_xyz, d_ans, d_desc;
-  std::vector<float> h_pts;
-  std::vector<int32_t> h_xyz;
-  std::vector<uint8_t> h_ans;
   // statistics
   std::vector<double> lat_all, lat_ins, lat_q, lat_occ;
   uint64_t completed = 0, n_ins = 0, n_q = 0, n_occ = 0, ticks = 0, rejected = 0;
@@ -200,16 +308,26 @@ int run_lookups(bxg_server_s* s, std::vector<Request*>& qs) {
     total += desc[k].n;
   }
   if (!total) return BXG_OK;
-  s->h_xyz.resize(3 * total);
-  for (size_t k = 0; k < look.size(); k++)
-    std::memcpy(s->h_xyz.data() + 3 * desc[k].begin, look[k]->coords.data(),
-                look[k]->coords.size() * 4);
+  size_t ans_cap = 0;
+  struct Answers {  // given back on every way out
+    HostPool& pool;
+    size_t& cap;
+    uint8_t* p;
+    ~Answers() {
+      if (p) pool.give(p, cap);
+    }
+  } held{s->pool, ans_cap, static_cast<uint8_t*>(s->pool.take(total, &ans_cap))};
+  uint8_t* const ans = held.p;
+  if (!ans) return BXG_ERR_CUDA;
   if (s->d_xyz.ensure(total * 12) != cudaSuccess || s->d_ans.ensure(total) != cudaSuccess ||
       s->d_desc.ensure(desc.size() * sizeof(QueryDesc)) != cudaSuccess) {
     cudaGetLastError();
     return BXG_ERR_CUDA;
   }
-  cudaMemcpyAsync(s->d_xyz.p, s->h_xyz.data(), total * 12, cudaMemcpyHostToDevice, s->stream);
+  for (size_t k = 0; k < look.size(); k++)
+    if (desc[k].n)
+      cudaMemcpyAsync(s->d_xyz.as<int32_t>() + 3 * desc[k].begin, look[k]->coords.data(),
+                      look[k]->coords.size() * 4, cudaMemcpyHostToDevice, s->stream);
   cudaMemcpyAsync(s->d_desc.p, desc.data(), desc.size() * sizeof(QueryDesc),
                   cudaMemcpyHostToDevice, s->stream);
   int sms = 0;
@@ -218,16 +336,14 @@ int run_lookups(bxg_server_s* s, std::vector<Request*>& qs) {
   k_query_multi<<<blocks, 256, 0, s->stream>>>(s->d_desc.as<QueryDesc>(), uint32_t(desc.size()),
                                                s->d_xyz.as<int32_t>(), total,
                                                s->d_ans.as<uint8_t>());
-  s->h_ans.resize(total);
-  cudaMemcpyAsync(s->h_ans.data(), s->d_ans.p, total, cudaMemcpyDeviceToHost, s->stream);
+  cudaMemcpyAsync(ans, s->d_ans.p, total, cudaMemcpyDeviceToHost, s->stream);
   const cudaError_t e = cudaStreamSynchronize(s->stream);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return BXG_ERR_CUDA;
   }
   for (size_t k = 0; k < look.size(); k++) {
-    look[k]->answers.assign(s->h_ans.begin() + desc[k].begin,
-                            s->h_ans.begin() + desc[k].begin + desc[k].n);
+    look[k]->answers.assign(ans + desc[k].begin, ans + desc[k].begin + desc[k].n);
     look[k]->status = BXG_OK;
   }
   s->lookups += total;
@@ -358,13 +474,11 @@ void worker_loop(bxg_server_s* s) {
         org.insert(org.end(), r->origin, r->origin + 3);
         mr.push_back(r->max_range);
       }
-      s->h_pts.resize(3 * off.back());
-      for (size_t k = 0; k < admit.size(); k++)
-        std::memcpy(s->h_pts.data() + 3 * off[k], admit[k]->mid->pts.data(),
-                    admit[k]->mid->pts.size() * 4);
+      std::vector<const float*> parts;
+      for (MapTick* mt : admit) parts.push_back(mt->mid->pts.data());
       std::vector<uint64_t> rc(admit.size(), 0);
-      st = bxg_batch_insert_f32(s->batch, ms.data(), ms.size(), s->h_pts.data(), off.data(),
-                                org.data(), mr.data(), rc.data());
+      st = batch_insert(s->batch, ms.data(), ms.size(), nullptr, parts.data(), off.data(),
+                        org.data(), mr.data(), rc.data());
       for (size_t k = 0; k < admit.size(); k++) {
         admit[k]->mid->status = st;
         admit[k]->mid->ray_cells = rc[k];
@@ -416,10 +530,8 @@ void worker_loop(bxg_server_s* s) {
           s->live.erase(r->ticket);
           delete r;
         } else {
-          r->pts.clear();
-          r->pts.shrink_to_fit();
-          r->coords.clear();
-          r->coords.shrink_to_fit();
+          r->pts.reset();
+          r->coords.reset();
         }
       };
       for (Request* r : before) finish(r);
@@ -444,6 +556,7 @@ void worker_loop(bxg_server_s* s) {
       if (idle_wait) wake = std::min(first_deadline, t1 + std::chrono::milliseconds(50));
     }
     s->cv_done.notify_all();
+    s->pool.refill();
   }
 }
 
@@ -452,6 +565,13 @@ double pct(std::vector<double> v, double p) {
   std::sort(v.begin(), v.end());
   const size_t k = std::min(v.size() - 1, size_t(p * (v.size() - 1) + 0.5));
   return v[k];
+}
+
+int no_memory(bxg_server_s* s, Request* r) {
+  delete r;
+  std::lock_guard<std::mutex> lk(s->mu);
+  s->err = "no host memory for the request's input";
+  return BXG_ERR_CUDA;
 }
 
 int submit(bxg_server_s* s, Request* r, uint64_t* ticket) {
@@ -560,7 +680,7 @@ int bxg_server_insert(bxg_server s, uint32_t map, const float* xyz, size_t n,
   r->kind = K_INSERT;
   r->map = map;
   r->discard = discard != 0;
-  r->pts.assign(xyz, xyz + 3 * n);
+  if (!r->pts.assign(&s->pool, xyz, 3 * n)) return no_memory(s, r);
   std::memcpy(r->origin, origin, 12);
   r->max_range = max_range;
   return submit(s, r, ticket);
@@ -574,7 +694,7 @@ int bxg_server_query(bxg_server s, uint32_t map, const int32_t* xyz, size_t n, i
   r->map = map;
   r->mode = mode;
   r->discard = discard != 0;
-  r->coords.assign(xyz, xyz + 3 * n);
+  if (!r->coords.assign(&s->pool, xyz, 3 * n)) return no_memory(s, r);
   return submit(s, r, ticket);
 }
 
