@@ -293,12 +293,6 @@ using namespace bxg;
 
 namespace {
 
-uint32_t next_pow2(uint64_t v) {
-  uint32_t p = 64;
-  while (p < v) p <<= 1;
-  return p;
-}
-
 int check_grid(bxg_grid g) { return g ? BXG_OK : BXG_ERR_INVALID_ARG; }
 
 // Test hook for the bounded waits: marks the inner-node slot of the leaf
@@ -353,7 +347,7 @@ struct Dedup {
   uint32_t cap = 0;
 };
 int build_dedup(MapCore* m, const int32_t* dxyz, uint32_t n, bool keep_max, bool need_min, Dedup* D) {
-  D->cap = next_pow2(uint64_t(n) * 2);
+  D->cap = dedup_entries(n);
   BXG_CUDA(m, m->s_dedup.ensure(size_t(D->cap) * 4));
   BXG_CUDA(m, m->s_ep.ensure(size_t(n) * 16));
   D->tab = m->s_dedup.as<uint32_t>();
@@ -846,7 +840,7 @@ constexpr uint32_t kNoAllocMaxItems = 1u << 17;             // 131072 items per 
 constexpr uint32_t kNoAllocBuckets = 2u * kNoAllocMaxItems;  // 262144 x 16 B = 4 MiB
 // the items take the upper half, the table's entries of 4 bytes a part of the lower
 static_assert(kNoAllocMaxItems * 16u <= kNoAllocBuckets * 8u, "items");
-static_assert(kNoAllocMaxItems * 2u * 4u <= kNoAllocBuckets * 8u, "table");
+static_assert(kNoAllocMaxItems * 4u * 4u <= kNoAllocBuckets * 8u, "table");
 
 static __device__ __align__(256) uint4 g_noalloc_dedup[kNoAllocBuckets];
 
@@ -900,7 +894,7 @@ extern "C" int bxg_grid_set_values_noalloc(bxg_grid g, const int32_t* d_xyz,
   uint4* tab = nullptr;
   int st = noalloc_table(m, &tab);
   if (st) return st;
-  const uint32_t cap = next_pow2(uint64_t(n) * 2);  // <= kNoAllocBuckets
+  const uint32_t cap = dedup_entries(n);  // at most the lower half
   uint32_t* words = reinterpret_cast<uint32_t*>(tab);
   int4* item = reinterpret_cast<int4*>(tab + kNoAllocBuckets / 2);
   BXG_CUDA(m, cudaMemsetAsync(words, 0xFF, size_t(cap) * 4, m->stream));
