@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(256, 8) k_tick_winners(const TickArgs* __restr
 // Tasks are equal shares of the rays (near cells) and segments of all scans, about four
 // per block, taken as blocks become free; at least one piece per thread, so that a small
 // tick reaches every SM (8 maps of 2-20 k points: 31 us; with shares of 2048 pieces 112 us).
-// 64 maps, 674 M cells: 1.47 ms (2.69 ms as a phase of the persistent kernel, with
+// 64 maps, 674 M cells: 1.33 ms (2.69 ms as a phase of the persistent kernel, with
 // segments found by a prefix per 256 rays), bound by instruction issue.
 __global__ void __launch_bounds__(kMarkThreads, kMarkBlocksPerSM) k_tick_mark(
     const TickArgs* __restrict__ argp, const TickScan* __restrict__ sc) {
@@ -268,8 +268,8 @@ __global__ void __launch_bounds__(kMarkThreads, kMarkBlocksPerSM) k_tick_mark(
       const uint32_t n = min(T.M.ctr[C_CAST], T.n);
       const uint32_t a = uint32_t(lo - pre[s]), b = uint32_t(stop - pre[s]);
       uint32_t visited = 0;
-      mark_scan(T.M, Q, A.cast + T.pt_begin, min(a, n), min(b, n), max(a, n) - n, max(b, n) - n,
-                kMarkThreads, kMarkThreads, T.ox, T.oy, T.oz, S, visited);
+      mark_scan(T.M, Q, A.cast + T.pt_begin, min(a, n), min(b, n),
+                max(a, n) - n + (threadIdx.x & ~31u), max(b, n) - n, kMarkThreads, kMarkThreads, T.ox, T.oy, T.oz, S, visited);
       visited = __reduce_add_sync(0xffffffffu, visited);
       if ((threadIdx.x & 31) == 0 && visited)
         atomicAdd(reinterpret_cast<unsigned long long*>(T.M.ctr + C_STATS) + S_VISITED,

@@ -84,20 +84,27 @@ __device__ __forceinline__ uint32_t apply_leaf_slot(const DMap& M, int lx, int l
 // the thread before it is in at the same step. A cell's coordinates come from
 // one fused multiply-add per axis:
 //
-//   n(k) = floor((2 k d + m) / (2 m)) = floor(k d/m + 1/2)
+//   n(k) = sign(d) floor((2 k |d| + m) / (2 m)) = sign(d) floor(k |d|/m + 1/2)
 //
-// and floor(fma(k, fl(d/m), 1/2 + 1/(4m))) is exactly that for k < 801 and
-// m <= 2047: the values (2 k d + m) / (2 m) are multiples of 1/(2m), so adding
+// and floor(fma(k, fl(d fl(1/m)), 1/2 + sign(d)/(4m))) is exactly that for k < 801
+// and m <= 2047: the values (2 k |d| + m) / (2 m) are multiples of 1/(2m), so adding
 // half of that keeps each 1/(4m) >= 1.2e-4 from the next integer, and the
-// error (k 2^-25 of the slope, 2^-15 of the rounded sum, 2^-25 of the offset)
-// stays below 5.5e-5. Longer rays divide in integers.
+// error (k 2^-24 of the slope, 2^-15 of the rounded sum, 2^-25 of the offset)
+// stays below 8e-5; for d < 0 the value is 1 more than the floor of k d/m - 1/2 -
+// 1/(4m), which is never an integer. (All d, m and k of the range: compared on a CPU.)
+// Added to 2^23 + the origin's cell and rounded down, the float's low bits are the
+// cell's coordinate: no conversion, sign or origin is left to apply, and the exponent's
+// bits are a constant in the address. Longer rays divide in integers.
 //
 // What bounds it: instruction issue, and for clouds of one narrow direction (a
 // depth frame) the ORs that meet in few words of L2. Kernel times on a GB300,
 // L2 warm, against tasks of rays whose segments were found by a prefix and a
 // search and walked with integer divisions (the form before): LiDAR 131k points,
-// 9.3 M cells, 25 us (62); depth 307k points, 10.5 M cells, 59 us (105); room
-// 60k points 18 us (30); 2k points 9.5 us (16). Before the near cells got blocks of their
+// 9.3 M cells, 24 us (62); depth 307k points, 10.5 M cells, 59 us (105); room
+// 60k points 18 us (30); 2k points 8.5 us (16). With the sign, the origin and the number
+// of cells applied at each step (18.9 M instructions for the LiDAR scan, now 16.2 M) and
+// no load ahead these were 25, 60, 18 and 9.9 us, and 64 maps in a batch 1.47 ms, now 1.33.
+// Before the near cells got blocks of their
 // own these were 28, 62, 20 and 14 us, of which without the far ORs 26, 39, 19
 // and 13 us, and with every lane's cells ORed, neighbours' too, 36, 65, 21 us. Measured and not
 // kept: rays sorted by direction and collected per block in shared memory, in
@@ -146,9 +153,9 @@ __device__ __forceinline__ uint32_t far_segments(const ScanCube& Q, uint32_t len
 
 // One thread's ray, as the marking needs it.
 struct MarkRay {
-  float sx, sy, sz, off;  // slopes |d| / m and the rounding offset
-  int gx, gy, gz;         // signs
-  uint32_t m;             // cells to mark; 0: none
+  float sx, sy, sz;  // slopes d / m
+  float fx, fy, fz;  // rounding offsets
+  uint32_t m;        // cells to mark; 0: none
   int dx, dy, dz;
   uint32_t len;
 };
@@ -164,58 +171,88 @@ __device__ __forceinline__ MarkRay mark_ray(const DMap& M, const ScanCube& Q, in
   r.m = r.len < kMarkMaxRay ? min(r.len, Q.kin) : 0u;
   if (r.len >= min(kMarkMaxRay, Q.kin) && !Q.open)
     set_err(M, ERR_SCRATCH);  // outside the cube: cannot happen for scan rays
-  const float fm = static_cast<float>(max(r.len, 1u));
-  r.sx = __fdiv_rn(static_cast<float>(abs(r.dx)), fm);
-  r.sy = __fdiv_rn(static_cast<float>(abs(r.dy)), fm);
-  r.sz = __fdiv_rn(static_cast<float>(abs(r.dz)), fm);
-  r.off = 0.5f + __fdiv_rn(0.25f, fm);
-  r.gx = r.dx < 0 ? -1 : 1;
-  r.gy = r.dy < 0 ? -1 : 1;
-  r.gz = r.dz < 0 ? -1 : 1;
+  const float inv = __frcp_rn(static_cast<float>(max(r.len, 1u)));
+  r.sx = static_cast<float>(r.dx) * inv;
+  r.sy = static_cast<float>(r.dy) * inv;
+  r.sz = static_cast<float>(r.dz) * inv;
+  r.fx = __fmaf_rn(r.dx < 0 ? -0.25f : 0.25f, inv, 0.5f);
+  r.fy = __fmaf_rn(r.dy < 0 ? -0.25f : 0.25f, inv, 0.5f);
+  r.fz = __fmaf_rn(r.dz < 0 ? -0.25f : 0.25f, inv, 0.5f);
   return r;
 }
 
-// Cell k of the ray, relative to its origin cell.
+// The float 2^23 + n has the bits kFloatInt + n (0 <= n < 2^23).
+constexpr uint32_t kFloatInt = 0x4B000000u;
+__device__ __forceinline__ float float_int(int n) { return 8388608.0f + static_cast<float>(n); }
+// floor of step f along an axis plus the integer that c = float_int() was made of.
+__device__ __forceinline__ uint32_t step_bits(float f, float s, float off, float c) {
+  return __float_as_uint(__fadd_rd(__fmaf_rn(f, s, off), c));
+}
+
+// Cell k of the ray, whose origin is the cell (qx, qy, qz).
 template <bool LONG>
-__device__ __forceinline__ void mark_cell(const MarkRay& r, uint32_t k, int& x, int& y, int& z) {
+__device__ __forceinline__ void mark_cell(const MarkRay& r, uint32_t k, int qx, int qy, int qz,
+                                          int& x, int& y, int& z) {
   if (LONG) {
     const uint32_t tm = 2u * r.len;
-    x = int((2u * k * uint32_t(abs(r.dx)) + r.len) / tm) * r.gx;
-    y = int((2u * k * uint32_t(abs(r.dy)) + r.len) / tm) * r.gy;
-    z = int((2u * k * uint32_t(abs(r.dz)) + r.len) / tm) * r.gz;
+    auto step = [&](int d) {
+      const int n = int((2u * k * uint32_t(abs(d)) + r.len) / tm);
+      return d < 0 ? -n : n;
+    };
+    x = qx + step(r.dx);
+    y = qy + step(r.dy);
+    z = qz + step(r.dz);
   } else {
     const float f = static_cast<float>(k);
-    x = int(__float_as_uint(__fadd_rd(__fmaf_rn(f, r.sx, r.off), 8388608.0f)) - 0x4B000000u) * r.gx;
-    y = int(__float_as_uint(__fadd_rd(__fmaf_rn(f, r.sy, r.off), 8388608.0f)) - 0x4B000000u) * r.gy;
-    z = int(__float_as_uint(__fadd_rd(__fmaf_rn(f, r.sz, r.off), 8388608.0f)) - 0x4B000000u) * r.gz;
+    x = int(step_bits(f, r.sx, r.fx, float_int(qx)) - kFloatInt);
+    y = int(step_bits(f, r.sy, r.fy, float_int(qy)) - kFloatInt);
+    z = int(step_bits(f, r.sz, r.fz, float_int(qz)) - kFloatInt);
   }
 }
 
-// Marks cells 0 .. n - 1 (n <= kNearCells) in the shared neighbourhood, whose
-// lowest cell is (wx, wy, wz) from the origin. The walk starts at cell rot: the
-// lanes of a warp are apart then, where they would all OR the origin's word.
+// Marks cells 0 .. n - 1 (1 <= n <= kNearCells) in the shared neighbourhood, where the
+// origin is the cell (nx, ny, nz). The walk starts at cell rot: the lanes of a warp are
+// apart then, where they would all OR the origin's word.
 template <bool LONG>
-__device__ __forceinline__ void mark_near(const MarkRay& r, uint32_t n, uint32_t rot, int wx,
-                                          int wy, int wz, uint32_t* sm) {
-  uint32_t cur = 0, acc = 0, k = rot;
-  for (uint32_t j = 0; j < n; ++j) {
-    int x, y, z;
-    mark_cell<LONG>(r, k, x, y, z);
-    const uint32_t X = uint32_t(x - wx), Y = uint32_t(y - wy), Z = uint32_t(z - wz);
-    const uint32_t w = (X >> 3) + kNearW * ((Y >> 2) + 2 * kNearW * Z);
+__device__ __forceinline__ void mark_near(const MarkRay& r, uint32_t n, uint32_t rot, int nx,
+                                          int ny, int nz, uint32_t* sm) {
+  // the constant that the words of the steps' bits carry
+  constexpr uint32_t kBias = LONG ? 0u
+                                  : (kFloatInt >> 3) + kNearW * (kFloatInt >> 2) +
+                                        2u * kNearW * kNearW * kFloatInt;
+  const float cx = float_int(nx), cy = float_int(ny), cz = float_int(nz);
+  uint32_t cur = 0, acc = 0;
+  auto put = [&](uint32_t X, uint32_t Y, uint32_t Z) {
+    const uint32_t w = (X >> 3) + kNearW * (Y >> 2) + 2 * kNearW * kNearW * Z;
     if (w != cur) {
-      if (acc) atomicOr(sm + cur, acc);
+      if (acc) atomicOr(sm + (cur - kBias), acc);
       acc = 0;
       cur = w;
     }
-    acc |= 1u << ((X & 7u) | ((Y & 3u) << 3));
-    k = k + 1 < n ? k + 1 : 0;
+    acc |= 1u << (((X & 7u) + (Y << 3)) & 31u);
+  };
+  if (LONG) {
+    uint32_t k = rot;
+    for (uint32_t j = 0; j < n; ++j) {
+      int x, y, z;
+      mark_cell<true>(r, k, nx, ny, nz, x, y, z);
+      put(uint32_t(x), uint32_t(y), uint32_t(z));
+      k = k + 1 < n ? k + 1 : 0;
+    }
+  } else {
+    const float last = static_cast<float>(n - 1);
+    float f = static_cast<float>(rot);
+    for (uint32_t j = 0; j < n; ++j) {
+      put(step_bits(f, r.sx, r.fx, cx), step_bits(f, r.sy, r.fy, cy),
+          step_bits(f, r.sz, r.fz, cz));
+      f = f < last ? f + 1.0f : 0.0f;
+    }
   }
-  if (acc) atomicOr(sm + cur, acc);
+  if (acc) atomicOr(sm + (cur - kBias), acc);
 }
 
-// Marks cells ka <= k < kb of each thread's ray in the bitmap (ka >= kb: none);
-// (qx, qy, qz): the origin in the cube. All lanes of the warp, unless LONG.
+// Marks cells ka <= k < kb (ka < kb) of each thread's ray in the bitmap, where the origin
+// is the cell (qx, qy, qz). All lanes of the warp, unless LONG.
 template <bool LONG>
 __device__ __forceinline__ void mark_far(const ScanCube& Q, const MarkRay& r, uint32_t ka,
                                          uint32_t kb, int qx, int qy, int qz) {
@@ -224,10 +261,12 @@ __device__ __forceinline__ void mark_far(const ScanCube& Q, const MarkRay& r, ui
   auto address = [&](uint32_t x, uint32_t y, uint32_t z) {
     return x + 8u * y + 64u * z + (x >> 3) * 504u + (y >> 3) * cy + (z >> 3) * cz;
   };
+  // the constant that the addresses of the steps' bits carry (a multiple of 32)
+  const uint32_t bias = LONG ? 0u : 73u * kFloatInt + (kFloatInt >> 3) * (504u + cy + cz);
   uint32_t cur = 0, acc = 0;
   auto put = [&](uint32_t a) {
     if ((a ^ cur) & ~31u) {
-      if (acc) red_or(Q.bits + (cur >> 5), acc);
+      if (acc) red_or(Q.bits + ((cur - bias) >> 5), acc);
       acc = 0;
       cur = a;
     }
@@ -236,30 +275,26 @@ __device__ __forceinline__ void mark_far(const ScanCube& Q, const MarkRay& r, ui
   if (LONG) {
     for (uint32_t k = ka; k < kb; ++k) {
       int x, y, z;
-      mark_cell<true>(r, k, x, y, z);
-      put(address(uint32_t(qx + x), uint32_t(qy + y), uint32_t(qz + z)));
+      mark_cell<true>(r, k, qx, qy, qz, x, y, z);
+      put(address(uint32_t(x), uint32_t(y), uint32_t(z)));
     }
   } else {
-    // 2^23 + n as a float has the bits 0x4B000000 + n
-    const uint32_t px = uint32_t(qx) - 0x4B000000u * uint32_t(r.gx),
-                   py = uint32_t(qy) - 0x4B000000u * uint32_t(r.gy),
-                   pz = uint32_t(qz) - 0x4B000000u * uint32_t(r.gz);
+    const float bx = float_int(qx), by = float_int(qy), bz = float_int(qz);
     const bool first = (threadIdx.x & 31) == 0;
-    const uint32_t steps = __reduce_max_sync(0xffffffffu, kb > ka ? kb - ka : 0u);
-    const float fe = static_cast<float>(kb);
+    const uint32_t steps = min(__reduce_max_sync(0xffffffffu, kb - ka), kSegCells);
+    // a thread whose segment is shorter than the warp's longest stays at its last cell
+    const float last = static_cast<float>(kb - 1);
     float f = static_cast<float>(ka);
-    for (uint32_t j = 0; j < steps; ++j, f += 1.0f) {
-      const uint32_t ix = __float_as_uint(__fadd_rd(__fmaf_rn(f, r.sx, r.off), 8388608.0f)),
-                     iy = __float_as_uint(__fadd_rd(__fmaf_rn(f, r.sy, r.off), 8388608.0f)),
-                     iz = __float_as_uint(__fadd_rd(__fmaf_rn(f, r.sz, r.off), 8388608.0f));
-      const uint32_t a = address(px + ix * uint32_t(r.gx), py + iy * uint32_t(r.gy),
-                                 pz + iz * uint32_t(r.gz));
-      const bool act = f < fe;
-      const uint32_t before = __shfl_up_sync(0xffffffffu, act ? a : kNone, 1);
-      if (act && (first || before != a)) put(a);
+    for (uint32_t j = 0; j < steps; ++j) {
+      const uint32_t a =
+          address(step_bits(f, r.sx, r.fx, bx), step_bits(f, r.sy, r.fy, by),
+                  step_bits(f, r.sz, r.fz, bz));
+      const uint32_t before = __shfl_up_sync(0xffffffffu, a, 1);
+      if (first || before != a) put(a);
+      f = fminf(f + 1.0f, last);
     }
   }
-  if (acc) red_or(Q.bits + (cur >> 5), acc);
+  if (acc) red_or(Q.bits + ((cur - bias) >> 5), acc);
 }
 
 // The roots between two cells (at most 32 apart on each axis) into the block's root bits.
@@ -283,8 +318,9 @@ struct MarkShared {
 };
 
 // A block's part of a scan's rays: the near cells of rays r, r + r_step, ... < r_end (r: the
-// first thread's), and the segments s, s + s_step, ... < s_end likewise (steps a multiple of
-// kMarkThreads). All threads of a block of kMarkThreads. Adds the cells walked to `visited`.
+// first thread's), and the segments s, s + s_step, ... < s_end of each warp's first lane (steps
+// a multiple of kMarkThreads). All threads of a block of kMarkThreads. Adds the cells walked to
+// `visited`.
 __device__ __forceinline__ void mark_scan(const DMap& M, const ScanCube& Q,
                                           const int4* __restrict__ cast, uint32_t r,
                                           uint32_t r_end, uint32_t s, uint32_t s_end,
@@ -295,6 +331,15 @@ __device__ __forceinline__ void mark_scan(const DMap& M, const ScanCube& Q,
   const int wx = ((qx >> 3) - kNearNB) * 8 - qx, wy = ((qy >> 3) - kNearNB) * 8 - qy,
             wz = ((qz >> 3) - kNearNB) * 8 - qz;
   const uint32_t root_words = cube_root_words(Q);
+  // a thread's next segment and its ray are loaded ahead of the one it walks; threads past
+  // the end go over the last segment again
+  auto segment = [&](uint32_t i) { return Q.segs[min(i + (threadIdx.x & 31), s_end - 1)]; };
+  uint32_t seg = 0;
+  int4 e = make_int4(0, 0, 0, 0);
+  if (s < s_end) {
+    seg = segment(s);
+    e = cast[seg >> 8];
+  }
   if (r < r_end)
     for (uint32_t t = threadIdx.x; t < kNearWords; t += kMarkThreads) S.near[t] = 0u;
   for (uint32_t t = threadIdx.x; t < root_words; t += kMarkThreads) S.roots[t] = 0u;
@@ -306,38 +351,39 @@ __device__ __forceinline__ void mark_scan(const DMap& M, const ScanCube& Q,
     const uint32_t n = min(q.m, kNearCells);
     const uint32_t rot = (threadIdx.x & 31) * n >> 5;
     if (q.len > kFmaMaxRay)
-      mark_near<true>(q, n, rot, wx, wy, wz, S.near);
+      mark_near<true>(q, n, rot, -wx, -wy, -wz, S.near);
     else
-      mark_near<false>(q, n, rot, wx, wy, wz, S.near);
+      mark_near<false>(q, n, rot, -wx, -wy, -wz, S.near);
     if (Q.segs) continue;
     for (uint32_t ka = kNearCells; ka < q.m; ka += kSegCells) {
       const uint32_t kb = min(ka + kSegCells, q.m);
       int ax, ay, az, bx, by, bz;
-      mark_cell<true>(q, ka, ax, ay, az);
-      mark_cell<true>(q, kb - 1, bx, by, bz);
+      mark_cell<true>(q, ka, qx, qy, qz, ax, ay, az);
+      mark_cell<true>(q, kb - 1, qx, qy, qz, bx, by, bz);
       mark_far<true>(Q, q, ka, kb, qx, qy, qz);
-      flag_roots(Q, qx + ax, qy + ay, qz + az, qx + bx, qy + by, qz + bz, S.roots);
+      flag_roots(Q, ax, ay, az, bx, by, bz, S.roots);
     }
   }
-  for (uint32_t i0 = s + (threadIdx.x & ~31u); i0 < s_end; i0 += s_step) {
-    const uint32_t i = i0 + (threadIdx.x & 31);
-    const uint32_t seg = i < s_end ? Q.segs[i] : 0u;
-    const MarkRay q = mark_ray(M, Q, cast[seg >> 8], ox, oy, oz);
+  while (s < s_end) {
+    const MarkRay q = mark_ray(M, Q, e, ox, oy, oz);
     const uint32_t ka = kNearCells + (seg & 255u) * kSegCells;
-    const uint32_t kb = i < s_end ? min(ka + kSegCells, q.m) : 0u;
-    int ax = 0, ay = 0, az = 0, bx = 0, by = 0, bz = 0;
+    const uint32_t kb = min(ka + kSegCells, q.m);
+    s += s_step;
+    if (s < s_end) {
+      seg = segment(s);
+      e = cast[seg >> 8];
+    }
+    int ax, ay, az, bx, by, bz;
     if (__any_sync(0xffffffffu, q.len > kFmaMaxRay)) {
-      if (kb) {
-        mark_cell<true>(q, ka, ax, ay, az);
-        mark_cell<true>(q, kb - 1, bx, by, bz);
-        mark_far<true>(Q, q, ka, kb, qx, qy, qz);
-      }
+      mark_cell<true>(q, ka, qx, qy, qz, ax, ay, az);
+      mark_cell<true>(q, kb - 1, qx, qy, qz, bx, by, bz);
+      mark_far<true>(Q, q, ka, kb, qx, qy, qz);
     } else {
-      mark_cell<false>(q, ka, ax, ay, az);
-      mark_cell<false>(q, kb - 1, bx, by, bz);
+      mark_cell<false>(q, ka, qx, qy, qz, ax, ay, az);
+      mark_cell<false>(q, kb - 1, qx, qy, qz, bx, by, bz);
       mark_far<false>(Q, q, ka, kb, qx, qy, qz);
     }
-    if (kb) flag_roots(Q, qx + ax, qy + ay, qz + az, qx + bx, qy + by, qz + bz, S.roots);
+    flag_roots(Q, ax, ay, az, bx, by, bz, S.roots);
   }
   __syncthreads();
   if (r < r_end) {

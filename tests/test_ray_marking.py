@@ -48,6 +48,20 @@ def _cloud(rng, lengths, res, origin):
     return (origin + (np.asarray(lengths)[:, None] + 0.3) * d * res).astype(np.float32)
 
 
+def test_signed_fma_gives_the_bresenham_cell():
+    """floor(fma(k, fl(d fl(1/m)), 1/2 + sign(d)/(4m))), the form with the sign in it."""
+    one, q, h = np.float32(1), np.float32(0.25), np.float64(0.5)
+    for m in list(range(1, 100)) + [255, 256, 257, 511, 769, 801, 1023, 1024, 1500, 2046, 2047]:
+        d = np.arange(-m, m + 1) if m < 100 else np.unique(np.concatenate(
+            [np.random.default_rng(m).integers(-m, m + 1, 400), [-m, 1 - m, -1, 0, 1, m - 1, m]]))
+        inv = one / np.float32(m)
+        s = (d.astype(np.float32) * inv).astype(np.float64)
+        off = (h + np.where(d < 0, -q, q).astype(np.float64) * np.float64(inv)).astype(np.float32)
+        k = np.arange(min(m, MAX_K))[:, None]
+        got = np.floor((k * s + off.astype(np.float64)).astype(np.float32)).astype(np.int64)
+        assert np.array_equal(got, np.sign(d) * ((2 * k * np.abs(d) + m) // (2 * m)))
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("res,max_range", [
     (0.1, 0.25),           # one root on each side of the origin's
