@@ -122,6 +122,13 @@ __device__ __forceinline__ uint4 ld_volatile4(const uint4* p) {
                : "memory");
   return v;
 }
+// Waits until the stream's kernels before this one are done and their writes are visible:
+// the first statement of a kernel that is launched with launch_after. Its pointers are not
+// declared const __restrict__ (the compiler could load through those before the wait).
+__device__ __forceinline__ void after_previous() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 __device__ __forceinline__ uint32_t ld_volatile(const uint32_t* p) {
   return *reinterpret_cast<const volatile uint32_t*>(p);
 }

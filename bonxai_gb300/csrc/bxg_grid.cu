@@ -51,9 +51,10 @@ __device__ __forceinline__ int3 coord_of(const int32_t* __restrict__ xyz, uint32
 // entry without a search, takes 7.2 us instead of 12.4.
 template <bool KEEP_MAX>
 __global__ void __launch_bounds__(256) k_dedup_insert(const __grid_constant__ DMap M,
-                                                      const int32_t* __restrict__ xyz, uint32_t n,
-                                                      uint32_t* tab, uint32_t tmask,
-                                                      int4* __restrict__ item, uint32_t* tab_min) {
+                                                      const int32_t* xyz, uint32_t n,
+                                                      uint32_t* tab, uint32_t tmask, int4* item,
+                                                      uint32_t* tab_min) {
+  after_previous();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int3 c = coord_of(xyz, i);
@@ -129,9 +130,9 @@ __device__ __forceinline__ uint32_t leaf_or_create(const DMap& M, uint32_t in, i
 // bucket) -> child -> value.
 template <int ESZ>
 __global__ void __launch_bounds__(256) k_set_values(const __grid_constant__ DMap M,
-                                                    const int4* __restrict__ item,
-                                                    const uint8_t* __restrict__ vals, uint32_t n,
-                                                    const uint32_t* __restrict__ tab) {
+                                                    const int4* item, const uint8_t* vals,
+                                                    uint32_t n, const uint32_t* tab) {
+  after_previous();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int4 c = item[i];
@@ -162,8 +163,9 @@ __global__ void k_was_on_first(const int4* __restrict__ item, uint32_t n,
 // setCellOn for the first item of each cell (bonxai.hpp:537-553): the default
 // is written only if the cell was off.
 template <int ESZ>
-__global__ void k_set_on(const __grid_constant__ DMap M, const int4* __restrict__ item, uint32_t n,
-                         const uint8_t* __restrict__ dflt, const uint32_t* __restrict__ tab) {
+__global__ void k_set_on(const __grid_constant__ DMap M, const int4* item, uint32_t n,
+                         const uint8_t* dflt, const uint32_t* tab) {
+  after_previous();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int4 c = item[i];
@@ -183,8 +185,9 @@ __global__ void k_set_on(const __grid_constant__ DMap M, const int4* __restrict_
 // setCellOff for the first item of each cell (bonxai.hpp:556-569). The value
 // is zeroed to keep the off-cells-hold-T{} invariant (not observable).
 template <int ESZ>
-__global__ void k_set_off(const __grid_constant__ DMap M, const int4* __restrict__ item, uint32_t n,
-                          const uint32_t* __restrict__ tab, uint8_t* out) {
+__global__ void k_set_off(const __grid_constant__ DMap M, const int4* item, uint32_t n,
+                          const uint32_t* tab, uint8_t* out) {
+  after_previous();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int4 c = item[i];
@@ -346,7 +349,9 @@ struct Dedup {
   uint32_t* tab_min = nullptr;
   uint32_t cap = 0;
 };
-int build_dedup(MapCore* m, const int32_t* dxyz, uint32_t n, bool keep_max, bool need_min, Dedup* D) {
+// The empty table of a batch of n. Before the kernel that makes the batch's coordinates, if
+// there is one: no memset then stands between it and k_dedup_insert.
+int clear_dedup(MapCore* m, uint32_t n, bool need_min, Dedup* D) {
   D->cap = dedup_entries(n);
   BXG_CUDA(m, m->s_dedup.ensure(size_t(D->cap) * 4));
   BXG_CUDA(m, m->s_ep.ensure(size_t(n) * 16));
@@ -360,13 +365,13 @@ int build_dedup(MapCore* m, const int32_t* dxyz, uint32_t n, bool keep_max, bool
     BXG_CUDA(m, cudaMemsetAsync(m->s_dedup2.p, 0xFF, size_t(D->cap) * 4, m->stream));
     D->tab_min = m->s_dedup2.as<uint32_t>();
   }
-  const unsigned blocks = (n + 255) / 256;
-  if (keep_max)
-    k_dedup_insert<true><<<blocks, 256, 0, m->stream>>>(m->dm, dxyz, n, D->tab, D->cap - 1, D->item,
-                                                        D->tab_min);
-  else
-    k_dedup_insert<false><<<blocks, 256, 0, m->stream>>>(m->dm, dxyz, n, D->tab, D->cap - 1,
-                                                         D->item, D->tab_min);
+  return BXG_OK;
+}
+
+// Enters the items into a table from clear_dedup.
+int build_dedup(MapCore* m, const int32_t* dxyz, uint32_t n, bool keep_max, const Dedup& D) {
+  launch_after(keep_max ? k_dedup_insert<true> : k_dedup_insert<false>, (n + 255) / 256, 256,
+               m->stream, m->dm, dxyz, n, D.tab, D.cap - 1, D.item, D.tab_min);
   BXG_LAUNCHED(m);
   return BXG_OK;
 }
@@ -380,20 +385,19 @@ void launch_set_values(MapCore* m, const int4* item, const uint8_t* vals, uint32
                        const uint32_t* tab) {
   const unsigned blocks = (n + 255) / 256;
   switch (m->dm.esz) {
-    case 0: k_set_values<0><<<blocks, 256, 0, m->stream>>>(m->dm, item, vals, n, tab); break;
-    case 1: k_set_values<1><<<blocks, 256, 0, m->stream>>>(m->dm, item, vals, n, tab); break;
-    case 2: k_set_values<2><<<blocks, 256, 0, m->stream>>>(m->dm, item, vals, n, tab); break;
-    case 4: k_set_values<4><<<blocks, 256, 0, m->stream>>>(m->dm, item, vals, n, tab); break;
-    default: k_set_values<8><<<blocks, 256, 0, m->stream>>>(m->dm, item, vals, n, tab); break;
+    case 0: launch_after(k_set_values<0>, blocks, 256, m->stream, m->dm, item, vals, n, tab); break;
+    case 1: launch_after(k_set_values<1>, blocks, 256, m->stream, m->dm, item, vals, n, tab); break;
+    case 2: launch_after(k_set_values<2>, blocks, 256, m->stream, m->dm, item, vals, n, tab); break;
+    case 4: launch_after(k_set_values<4>, blocks, 256, m->stream, m->dm, item, vals, n, tab); break;
+    default: launch_after(k_set_values<8>, blocks, 256, m->stream, m->dm, item, vals, n, tab); break;
   }
 }
 
 int grid_set_values_dev(bxg_grid g, const int32_t* dxyz, const void* dvals, uint32_t n,
-                        uint8_t* was_on) {
+                        uint8_t* was_on, const Dedup& D) {
   MapCore* m = &g->core;
   const bool want_was = was_on != nullptr;
-  Dedup D;
-  int st = build_dedup(m, dxyz, n, true, want_was, &D);
+  int st = build_dedup(m, dxyz, n, true, D);
   if (st) return st;
   uint8_t* pre = want_was ? pre_bytes(m, D.cap, true) : nullptr;
   const unsigned blocks = (n + 255) / 256;
@@ -439,10 +443,13 @@ int grid_set_at_points(bxg_grid g, const PT* xyz, size_t stride, size_t n, const
   // a pass of its own: in the dedup kernel, which reads coordinates of other items too, the
   // double-precision products cost more (50 k points: 17.4 us, against 3.4 + 8.9)
   BXG_CUDA(m, m->s_out.ensure(n * 12));
+  Dedup D;
+  st = clear_dedup(m, uint32_t(n), false, &D);
+  if (st) return st;
   k_pos_to_coord<PT><<<unsigned((n + 255) / 256), 256, 0, m->stream>>>(
       static_cast<const uint8_t*>(dpts), stride, uint32_t(n), m->inv_res, m->s_out.as<int32_t>());
   BXG_LAUNCHED(m);
-  return grid_set_values_dev(g, m->s_out.as<int32_t>(), dvals, uint32_t(n), nullptr);
+  return grid_set_values_dev(g, m->s_out.as<int32_t>(), dvals, uint32_t(n), nullptr, D);
 }
 
 }  // namespace
@@ -504,8 +511,11 @@ int bxg_grid_set_values(bxg_grid g, const int32_t* xyz, const void* values, size
   if (st) return st;
   st = stage_in(m, m->s_in2, values, n * size_t(m->dm.esz), &dvals);
   if (st) return st;
+  Dedup D;
+  st = clear_dedup(m, uint32_t(n), was_on != nullptr, &D);
+  if (st) return st;
   return grid_set_values_dev(g, static_cast<const int32_t*>(dxyz), dvals, uint32_t(n),
-                             was_on);
+                             was_on, D);
 }
 
 int bxg_grid_set_values_at_points_f32(bxg_grid g, const float* xyz, size_t stride, size_t n,
@@ -613,7 +623,9 @@ int bxg_grid_set_cells_on(bxg_grid g, const int32_t* xyz, size_t n, const void* 
     if (st) return st;
   }
   Dedup D;
-  st = build_dedup(m, static_cast<const int32_t*>(dxyz), uint32_t(n), false, false, &D);
+  st = clear_dedup(m, uint32_t(n), false, &D);
+  if (st) return st;
+  st = build_dedup(m, static_cast<const int32_t*>(dxyz), uint32_t(n), false, D);
   if (st) return st;
   BXG_CUDA(m, m->s_dedup2.ensure(size_t(D.cap)));
   uint8_t* pre = pre_bytes(m, D.cap, false);
@@ -626,11 +638,11 @@ int bxg_grid_set_cells_on(bxg_grid g, const int32_t* xyz, size_t n, const void* 
   st = run_with_growth(m, [&]() -> int {
     const uint32_t n32 = uint32_t(n);
     switch (esz) {
-      case 0: k_set_on<0><<<blocks, 256, 0, m->stream>>>(m->dm, D.item, n32, d, D.tab); break;
-      case 1: k_set_on<1><<<blocks, 256, 0, m->stream>>>(m->dm, D.item, n32, d, D.tab); break;
-      case 2: k_set_on<2><<<blocks, 256, 0, m->stream>>>(m->dm, D.item, n32, d, D.tab); break;
-      case 4: k_set_on<4><<<blocks, 256, 0, m->stream>>>(m->dm, D.item, n32, d, D.tab); break;
-      default: k_set_on<8><<<blocks, 256, 0, m->stream>>>(m->dm, D.item, n32, d, D.tab); break;
+      case 0: launch_after(k_set_on<0>, blocks, 256, m->stream, m->dm, D.item, n32, d, D.tab); break;
+      case 1: launch_after(k_set_on<1>, blocks, 256, m->stream, m->dm, D.item, n32, d, D.tab); break;
+      case 2: launch_after(k_set_on<2>, blocks, 256, m->stream, m->dm, D.item, n32, d, D.tab); break;
+      case 4: launch_after(k_set_on<4>, blocks, 256, m->stream, m->dm, D.item, n32, d, D.tab); break;
+      default: launch_after(k_set_on<8>, blocks, 256, m->stream, m->dm, D.item, n32, d, D.tab); break;
     }
     BXG_LAUNCHED(m);
     return BXG_OK;
@@ -660,7 +672,9 @@ int bxg_grid_set_cells_off(bxg_grid g, const int32_t* xyz, size_t n, uint8_t* wa
   int st = stage_in(m, m->s_in, xyz, n * 12, &dxyz);
   if (st) return st;
   Dedup D;
-  st = build_dedup(m, static_cast<const int32_t*>(dxyz), uint32_t(n), false, false, &D);
+  st = clear_dedup(m, uint32_t(n), false, &D);
+  if (st) return st;
+  st = build_dedup(m, static_cast<const int32_t*>(dxyz), uint32_t(n), false, D);
   if (st) return st;
   void* dout = nullptr;
   st = stage_out(m, m->s_out, was_on, n, &dout);
@@ -669,11 +683,11 @@ int bxg_grid_set_cells_off(bxg_grid g, const int32_t* xyz, size_t n, uint8_t* wa
   uint8_t* o = static_cast<uint8_t*>(dout);
   const uint32_t n32 = uint32_t(n);
   switch (m->dm.esz) {
-    case 0: k_set_off<0><<<blocks, 256, 0, m->stream>>>(m->dm, D.item, n32, D.tab, o); break;
-    case 1: k_set_off<1><<<blocks, 256, 0, m->stream>>>(m->dm, D.item, n32, D.tab, o); break;
-    case 2: k_set_off<2><<<blocks, 256, 0, m->stream>>>(m->dm, D.item, n32, D.tab, o); break;
-    case 4: k_set_off<4><<<blocks, 256, 0, m->stream>>>(m->dm, D.item, n32, D.tab, o); break;
-    default: k_set_off<8><<<blocks, 256, 0, m->stream>>>(m->dm, D.item, n32, D.tab, o); break;
+    case 0: launch_after(k_set_off<0>, blocks, 256, m->stream, m->dm, D.item, n32, D.tab, o); break;
+    case 1: launch_after(k_set_off<1>, blocks, 256, m->stream, m->dm, D.item, n32, D.tab, o); break;
+    case 2: launch_after(k_set_off<2>, blocks, 256, m->stream, m->dm, D.item, n32, D.tab, o); break;
+    case 4: launch_after(k_set_off<4>, blocks, 256, m->stream, m->dm, D.item, n32, D.tab, o); break;
+    default: launch_after(k_set_off<8>, blocks, 256, m->stream, m->dm, D.item, n32, D.tab, o); break;
   }
   BXG_LAUNCHED(m);
   if (dout) {

@@ -125,11 +125,11 @@ __global__ void k_endpoints_kind(const __grid_constant__ DMap M, const double* _
 }
 
 // The lowest-index point of each endpoint cell (winners_block).
-__global__ void __launch_bounds__(256) k_winners(const __grid_constant__ DMap M, const int4* __restrict__ ep, uint32_t n,
-                          const uint4* __restrict__ tab, uint32_t tmask, int ox, int oy, int oz,
-                          int32_t u, Opts o, int4* __restrict__ cast, uint32_t cast_cap,
-                          const __grid_constant__ ScanCube Q) {
+__global__ void __launch_bounds__(256) k_winners(const __grid_constant__ DMap M, int4* ep, uint32_t n,
+                          uint4* tab, uint32_t tmask, int ox, int oy, int oz, int32_t u, Opts o,
+                          int4* cast, uint32_t cast_cap, const __grid_constant__ ScanCube Q) {
   __shared__ WinnersShared S;
+  after_previous();
   winners_block(M, ep, n, blockIdx.x * blockDim.x + threadIdx.x, tab, tmask, ox, oy, oz, u, o,
                 cast, cast_cap, Q, S);
 }
@@ -197,9 +197,9 @@ __global__ void __launch_bounds__(U == 2 ? 256 : 1024, U == 2 ? 3 : 1) k_rays(co
 // table, for the next scan.
 __global__ void __launch_bounds__(kMarkThreads, kMarkBlocksPerSM) k_mark(
     const __grid_constant__ DMap M, const __grid_constant__ ScanCube Q,
-    const int4* __restrict__ cast, uint32_t cast_cap, int ox, int oy, int oz,
-    uint4* __restrict__ tab, uint32_t tab_n) {
+    int4* cast, uint32_t cast_cap, int ox, int oy, int oz, uint4* tab, uint32_t tab_n) {
   __shared__ MarkShared S;
+  after_previous();
   for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < tab_n; t += gridDim.x * blockDim.x)
     tab[t] = make_uint4(kNone, kNone, kNone, kNone);
   const uint32_t n_cast = min(ld_volatile(M.ctr + C_CAST), cast_cap);
@@ -230,6 +230,7 @@ __global__ void __launch_bounds__(256, 4) k_apply_rays(const __grid_constant__ D
                                                     int32_t miss, int32_t cmin) {
   __shared__ uint32_t pre[kRootFlagWords], sums[kApplyWarps];
   __shared__ ApplyShared S;
+  after_previous();
   const uint32_t n_roots = apply_roots(Q, pre, sums);
   const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   uint32_t updated = 0;
@@ -244,9 +245,9 @@ __global__ void __launch_bounds__(256, 4) k_apply_rays(const __grid_constant__ D
 // The parts of the scan's rays that the cube does not hold (tail_rays).
 __global__ void __launch_bounds__(256) k_tail(const __grid_constant__ DMap M,
                                               const __grid_constant__ ScanCube Q,
-                                              const int4* __restrict__ cast, uint32_t cast_cap,
-                                              int ox, int oy, int oz, int32_t u, int32_t miss,
-                                              int32_t cmin) {
+                                              int4* cast, uint32_t cast_cap, int ox, int oy,
+                                              int oz, int32_t u, int32_t miss, int32_t cmin) {
+  after_previous();
   uint32_t visited = 0, updated = 0;
   tail_rays(M, Q, cast, cast_cap, (blockIdx.x * blockDim.x + threadIdx.x) >> 5,
             (gridDim.x * blockDim.x) >> 5, ox, oy, oz, u, miss, cmin, visited, updated);
@@ -357,10 +358,9 @@ int endpoint_phase(bxg_pmap_s* pm, uint32_t n, int ox, int oy, int oz, const Sca
   launch_ep(blocks, m->s_ep.as<int4>(), m->s_dedup.as<uint4>(), tcap - 1);
   BXG_LAUNCHED(m);
   record(pm, 1);
-  k_winners<<<blocks, 256, 0, m->stream>>>(m->dm, m->s_ep.as<int4>(), n, m->s_dedup.as<uint4>(),
-                                           tcap - 1, ox, oy, oz, pm->update_count, opts_of(pm),
-                                           m->s_cast.as<int4>(), uint32_t(m->s_cast.cap / 16),
-                                           cube);
+  launch_after(k_winners, blocks, 256, m->stream, m->dm, m->s_ep.as<int4>(), n,
+               m->s_dedup.as<uint4>(), tcap - 1, ox, oy, oz, pm->update_count, opts_of(pm),
+               m->s_cast.as<int4>(), uint32_t(m->s_cast.cap / 16), cube);
   BXG_LAUNCHED(m);
   record(pm, 2);
   pm->cast_ub = need;
@@ -527,20 +527,21 @@ int launch_rays(bxg_pmap_s* pm, int ox, int oy, int oz) {
       const unsigned mblocks = unsigned(
           std::min<uint64_t>(uint64_t(m->sm_count) * kMarkBlocksPerSM,
                              (pieces + kMarkThreads - 1) / kMarkThreads));
-      k_mark<<<mblocks, kMarkThreads, 0, m->stream>>>(m->dm, Q, m->s_cast.as<int4>(), ccap, ox,
-                                                      oy, oz, m->s_dedup.as<uint4>(), tab_n);
+      launch_after(k_mark, mblocks, kMarkThreads, m->stream, m->dm, Q, m->s_cast.as<int4>(), ccap,
+                   ox, oy, oz, m->s_dedup.as<uint4>(), tab_n);
       BXG_LAUNCHED(m);
       // the marked roots are at most those of the cube, or of the rays' pieces
       const uint64_t rows = 16 * std::min<uint64_t>(uint64_t(Q.SR) * Q.SR * Q.SR, 8 * pieces);
       const unsigned ablocks =
           unsigned(std::min<uint64_t>(uint64_t(m->sm_count) * 12, (rows + 7) / 8));
-      k_apply_rays<<<ablocks, 256, 0, m->stream>>>(m->dm, Q, pm->update_count, o.miss, o.cmin);
+      launch_after(k_apply_rays, ablocks, 256, m->stream, m->dm, Q, pm->update_count, o.miss,
+                   o.cmin);
       BXG_LAUNCHED(m);
       if (Q.open) {
         const unsigned tblocks = unsigned(std::min<uint64_t>(
             uint64_t(m->sm_count) * 8, (pm->cast_ub * kTailPieces + 7) / 8));
-        k_tail<<<tblocks, 256, 0, m->stream>>>(m->dm, Q, m->s_cast.as<int4>(), ccap, ox, oy, oz,
-                                               pm->update_count, o.miss, o.cmin);
+        launch_after(k_tail, tblocks, 256, m->stream, m->dm, Q, m->s_cast.as<int4>(), ccap, ox,
+                     oy, oz, pm->update_count, o.miss, o.cmin);
         BXG_LAUNCHED(m);
       }
       m->dedup_clean = std::max(m->dedup_clean, tab_n);
