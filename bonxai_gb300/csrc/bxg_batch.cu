@@ -59,7 +59,7 @@ struct TickScan {
   int32_t ox, oy, oz, u;
   Opts o;
   unsigned long long pt_begin;   // first point of this scan in the tick's arrays
-  unsigned long long tab_begin;  // first bucket of this scan's dedup table
+  unsigned long long tab_begin;  // of this scan's dedup table, in 16-byte units
   uint32_t n;                    // points
   uint32_t tmask;                // dedup table size - 1
   int32_t keep_nonfinite;
@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(256) k_tick_endpoints(const TickArgs* __restri
       e = compute_endpoint<float>(p, S.fx, S.fy, S.fz, S.max_range, S.mr2, S.inv_res,
                                   S.keep_nonfinite != 0, &S.fast);
     }
-    endpoint_enter(S.M, e, i, A.tab + S.tab_begin, S.tmask);
+    endpoint_enter(S.M, e, i, A.tab + S.tab_begin, S.tmask, dedup_key(S.Q));
     if (i < S.n) A.ep[S.pt_begin + i] = e;
   }
 }
@@ -418,7 +418,7 @@ __global__ void __launch_bounds__(256, U == 2 ? 3 : 4) k_tick(const TickArgs* __
     A.ep[i] = e;
     if (e.w != EP_SKIP)
       dedup_min_insert(A.tab + S.tab_begin, S.tmask, e.x, e.y, e.z,
-                       static_cast<uint32_t>(i - S.pt_begin), S.M);
+                       static_cast<uint32_t>(i - S.pt_begin), S.M, DedupKey{});
   }
   if (!grid_barrier(A.bar, A.err)) return;
   stamp(2);
@@ -435,7 +435,7 @@ __global__ void __launch_bounds__(256, U == 2 ? 3 : 4) k_tick(const TickArgs* __
       const TickScan& S = sc[s];
       e = A.ep[i];
       valid = e.w != EP_SKIP;
-      if (valid && dedup_lookup(A.tab + S.tab_begin, S.tmask, e.x, e.y, e.z) ==
+      if (valid && dedup_lookup(A.tab + S.tab_begin, S.tmask, e.x, e.y, e.z, DedupKey{}) ==
                        static_cast<uint32_t>(i - S.pt_begin))
         add = winner_apply(S.M, e, kPending, S.u, S.o);
     }
@@ -752,8 +752,6 @@ int batch_insert(bxg_batch b, const bxg_pmap* maps, size_t n_scans, const float*
   A.n_roots = reinterpret_cast<uint32_t*>(meta + kOffRoots);
   A.n_scans = uint32_t(n_scans);
   A.total_points = total;
-  A.total_tab = tab_total;
-  uint64_t tb = 0;
   for (size_t s = 0; s < n_scans; s++) {
     bxg_pmap_s* pm = maps[s];
     TickScan& S = b->h_scans[s];
@@ -774,10 +772,6 @@ int batch_insert(bxg_batch b, const bxg_pmap* maps, size_t n_scans, const float*
                pm->opt.clamp_max_log};
     S.pt_begin = offsets[s];
     S.n = uint32_t(offsets[s + 1] - offsets[s]);
-    const uint32_t tcap = dedup_entries(S.n);
-    S.tab_begin = tb;
-    S.tmask = tcap - 1;
-    tb += tcap;
     S.keep_nonfinite = (pm->core.flags & BXG_FLAG_KEEP_NONFINITE) ? 1 : 0;
   }
   // The two-phase ray update when every map can have its cube bitmap (each
@@ -818,6 +812,15 @@ int batch_insert(bxg_batch b, const bxg_pmap* maps, size_t n_scans, const float*
       if (has_segs[s]) S.Q.segs = b->segs.as<uint32_t>() + seg0[s];
       if (S.Q.open) S.Q.tails = b->tails.as<uint32_t>() + S.pt_begin;
     }
+  }
+  A.total_tab = 0;  // 16-byte units
+  for (size_t s = 0; s < n_scans; s++) {
+    TickScan& S = b->h_scans[s];
+    if (!mark) S.Q = ScanCube{};
+    const uint32_t tcap = dedup_entries(S.n);
+    S.tab_begin = A.total_tab;
+    S.tmask = tcap - 1;
+    A.total_tab += dedup_key(S.Q).packed ? tcap / 2 : tcap;
   }
   b->back_bytes = kBackBytes;
   const size_t param_bytes = 256 + n_scans * sizeof(TickScan);

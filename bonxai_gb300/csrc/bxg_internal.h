@@ -89,10 +89,10 @@ struct MapCore {
 
   // scratch
   DevBuf s_in, s_in2, s_out, s_out2, s_dedup, s_dedup2, s_ep, s_cast, s_tmp;
-  // entries of s_dedup known to be empty, from index 0 (the ray kernel clears
+  // 16-byte units of s_dedup known to be empty, from 0 (the ray phase clears
   // the table the last endpoint phase used, so the next one needs no memset)
   uint32_t dedup_clean = 0;
-  uint32_t dedup_used = 0;  // entries the last endpoint phase used
+  uint32_t dedup_used = 0;  // 16-byte units that the last endpoint phase used
   DevBuf s_dir;             // leaf directory of the ray kernel (bxg_scan.cuh)
 
   std::string err;
@@ -204,7 +204,8 @@ int run_with_growth(MapCore* m, F&& body) {
 // Entries of the endpoint dedup table of a scan of n points: a power of two, at least 2 n
 // and up to 16 n in small scans. A thread probes with one CAS after the other, about 1 us
 // each, and a small scan waits for the longest of the chains, while a large one has many
-// points per cell and pays for clearing its table. Endpoints at 2, 4, 8, 16 entries per
+// points per cell and pays for clearing its table. With entries of 16 bytes (dedup_key: now
+// 8 in most scans), endpoints at 2, 4, 8, 16 entries per
 // point: 2k points 10.2, 6.2, 5.3, 4.9 us; 60k room 11.6, 8.9, 8.3, 7.7 us with 17.4, 17.3,
 // 17.6, 19.6 us for k_mark, which clears it; 131k LiDAR 9.1, 7.6, 7.2, 7.2 with 24.9, 25.9,
 // 26.3, 27.6; 64 maps of 10-500 k points 264, 250, 248, 245 us with 55, 110, 219, 440 us to

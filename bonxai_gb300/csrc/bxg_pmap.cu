@@ -58,7 +58,7 @@ __global__ void k_endpoints(const __grid_constant__ DMap M, const uint8_t* __res
                             double fx, double fy, double fz, double max_range, double mr2,
                             double inv_res, int keep_nonfinite, int4* __restrict__ ep,
                             uint4* tab, uint32_t tmask, int zero_stats, EpFast F,
-                            uint32_t* roots, uint32_t root_words) {
+                            uint32_t* roots, uint32_t root_words, DedupKey K) {
   zero_scan_stats(M, zero_stats, roots, root_words);
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   int4 e = make_int4(0, 0, 0, EP_SKIP);
@@ -66,7 +66,7 @@ __global__ void k_endpoints(const __grid_constant__ DMap M, const uint8_t* __res
     const PT* p = reinterpret_cast<const PT*>(pts + size_t(i) * stride);
     e = compute_endpoint<PT>(p, fx, fy, fz, max_range, mr2, inv_res, keep_nonfinite != 0, &F);
   }
-  endpoint_enter(M, e, i, tab, tmask);
+  endpoint_enter(M, e, i, tab, tmask, K);
   if (i < n) ep[i] = e;
 }
 
@@ -92,7 +92,7 @@ __global__ void k_endpoints_sensor(const __grid_constant__ DMap M, const uint8_t
                                    double max_range, double mr2, double inv_res,
                                    int4* __restrict__ ep, uint4* tab, uint32_t tmask,
                                    int zero_stats, EpFast F, uint32_t* roots,
-                                   uint32_t root_words) {
+                                   uint32_t root_words, DedupKey K) {
   zero_scan_stats(M, zero_stats, roots, root_words);
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -105,7 +105,7 @@ __global__ void k_endpoints_sensor(const __grid_constant__ DMap M, const uint8_t
   const float w[3] = {xf_row(xf, 0, x, y, z), xf_row(xf, 1, x, y, z), xf_row(xf, 2, x, y, z)};
   const int4 e = compute_endpoint<float>(w, fx, fy, fz, max_range, mr2, inv_res, true, &F);
   ep[i] = e;
-  if (e.w != EP_SKIP) dedup_min_insert(tab, tmask, e.x, e.y, e.z, i, M);
+  if (e.w != EP_SKIP) dedup_min_insert(tab, tmask, e.x, e.y, e.z, i, M, K);
 }
 
 // addHitPoint / addMissPoint batches: double points with a given kind, or a
@@ -121,7 +121,7 @@ __global__ void k_endpoints_kind(const __grid_constant__ DMap M, const double* _
   const int cy = __double2int_rd(__dmul_rn(pts[3 * i + 1], inv_res));
   const int cz = __double2int_rd(__dmul_rn(pts[3 * i + 2], inv_res));
   ep[i] = make_int4(cx, cy, cz, kind);
-  dedup_min_insert(tab, tmask, cx, cy, cz, i, M);
+  dedup_min_insert(tab, tmask, cx, cy, cz, i, M, DedupKey{});
 }
 
 // The lowest-index point of each endpoint cell (winners_block).
@@ -346,14 +346,15 @@ int endpoint_phase(bxg_pmap_s* pm, uint32_t n, int ox, int oy, int oz, const Sca
   const uint32_t tcap = dedup_entries(n);
   BXG_CUDA(m, m->s_ep.ensure(size_t(n) * 16));
   const void* old_tab = m->s_dedup.p;
-  BXG_CUDA(m, m->s_dedup.ensure(size_t(tcap) * 16));
+  const uint32_t tab_n = dedup_key(cube).packed ? tcap / 2 : tcap;  // 16-byte units
+  BXG_CUDA(m, m->s_dedup.ensure(size_t(tab_n) * 16));
   if (m->s_dedup.p != old_tab) m->dedup_clean = 0;
   // the ray list persists across add-batches until updateFreeCells
   const uint64_t need = pm->cast_ub + n;
   BXG_CUDA(m, m->s_cast.ensure_keep(need * 16, pm->cast_ub * 16, m->stream));
-  if (m->dedup_clean < tcap) launch_dedup_clear(m, m->s_dedup.as<uint4>(), tcap);
+  if (m->dedup_clean < tab_n) launch_dedup_clear(m, m->s_dedup.as<uint4>(), tab_n);
   m->dedup_clean = 0;
-  m->dedup_used = std::max(m->dedup_used, tcap);
+  m->dedup_used = std::max(m->dedup_used, tab_n);
   const unsigned blocks = (n + 255) / 256;
   launch_ep(blocks, m->s_ep.as<int4>(), m->s_dedup.as<uint4>(), tcap - 1);
   BXG_LAUNCHED(m);
@@ -721,6 +722,7 @@ int insert_impl(bxg_pmap m_, const PT* xyz, size_t stride, size_t n, const PT* o
     }
     const uint32_t root_words = cube.roots ? cube_root_words(cube) : 0;
     const int zero = ZERO_STATS | ZERO_RAYS | (pm->cast_ub == 0 ? ZERO_CAST : 0);
+    const DedupKey key = dedup_key(cube);
     EpFast fast = make_ep_fast(fx, fy, fz, max_range, m->inv_res);
     if (sizeof(PT) != 4) fast.on = 0;
     st = endpoint_phase(pm, uint32_t(n), o[0], o[1], o[2], cube,
@@ -729,12 +731,12 @@ int insert_impl(bxg_pmap m_, const PT* xyz, size_t stride, size_t n, const PT* o
                             k_endpoints_sensor<<<blocks, 256, 0, m->stream>>>(
                                 m->dm, static_cast<const uint8_t*>(dpts), stride, uint32_t(n),
                                 *xf, fx, fy, fz, max_range, mr2, m->inv_res, ep, tab, tmask, zero,
-                                fast, cube.roots, root_words);
+                                fast, cube.roots, root_words, key);
                           else
                             k_endpoints<PT><<<blocks, 256, 0, m->stream>>>(
                                 m->dm, static_cast<const uint8_t*>(dpts), stride, uint32_t(n), fx,
                                 fy, fz, max_range, mr2, m->inv_res, keep, ep, tab, tmask, zero,
-                                fast, cube.roots, root_words);
+                                fast, cube.roots, root_words, key);
                         });
     if (st) return st;
   }

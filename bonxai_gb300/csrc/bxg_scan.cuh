@@ -35,9 +35,47 @@ __device__ __forceinline__ bool finite3(double a, double b, double c) {
   return isfinite(a) && isfinite(b) && isfinite(c);
 }
 
-// Lowest index per endpoint cell (scratch table, all-ones = empty).
+// Lowest index per endpoint cell (scratch table, all-ones = empty). A scan whose endpoints
+// lie in a cube of 2^11 cells a side from (x0, y0, z0) packs an entry into 64 bits: 33 of
+// the cell in the cube, 31 of the index. Others have entries of a cell and an index, 128
+// bits.
+struct DedupKey {
+  int x0, y0, z0;
+  uint32_t packed;
+};
+constexpr unsigned long long kPackedEmpty = ~0ull;
+constexpr uint32_t kPackedIndex = 0x7FFFFFFFu;
+
+// The entry of a cell without its index; false: outside the cube.
+__device__ __forceinline__ bool packed_key(const DedupKey& K, int x, int y, int z,
+                                           unsigned long long& key) {
+  const uint32_t rx = uint32_t(x - K.x0), ry = uint32_t(y - K.y0), rz = uint32_t(z - K.z0);
+  key = ((static_cast<unsigned long long>(rz) << 22) | (ry << 11) | rx) << 31;
+  return (rx | ry | rz) < 2048u;
+}
+
 __device__ __forceinline__ void dedup_min_insert(uint4* tab, uint32_t tmask, int x, int y, int z,
-                                                 uint32_t i, const DMap& M) {
+                                                 uint32_t i, const DMap& M, const DedupKey& K) {
+  if (K.packed) {
+    unsigned long long* t = reinterpret_cast<unsigned long long*>(tab);
+    unsigned long long key;
+    if (!packed_key(K, x, y, z, key)) {
+      set_err(M, ERR_SCRATCH);  // outside the cube: cannot happen for scan rays
+      return;
+    }
+    const unsigned long long mine = key | i;
+    uint32_t h = cell_hash(x, y, z) & tmask;
+    for (uint32_t p = 0; p <= tmask; ++p, h = (h + 1) & tmask) {
+      const unsigned long long old = atomicCAS(t + h, kPackedEmpty, mine);
+      if (old == kPackedEmpty) return;
+      if (((old ^ mine) >> 31) == 0ull) {
+        if (mine < old) atomicMin(t + h, mine);
+        return;
+      }
+    }
+    set_err(M, ERR_SCRATCH);
+    return;
+  }
   const uint4 kEmpty = make_uint4(kNone, kNone, kNone, kNone);
   const uint4 mine = make_uint4(uint32_t(x), uint32_t(y), uint32_t(z), i);
   uint32_t h = cell_hash(x, y, z) & tmask;
@@ -53,7 +91,19 @@ __device__ __forceinline__ void dedup_min_insert(uint4* tab, uint32_t tmask, int
 }
 
 __device__ __forceinline__ uint32_t dedup_lookup(const uint4* tab, uint32_t tmask, int x, int y,
-                                                 int z) {
+                                                 int z, const DedupKey& K) {
+  if (K.packed) {
+    const unsigned long long* t = reinterpret_cast<const unsigned long long*>(tab);
+    unsigned long long key;
+    packed_key(K, x, y, z, key);
+    uint32_t h = cell_hash(x, y, z) & tmask;
+    for (uint32_t p = 0; p <= tmask; ++p, h = (h + 1) & tmask) {
+      const unsigned long long b = t[h];
+      if (b == kPackedEmpty) return kNone;
+      if (((b ^ key) >> 31) == 0ull) return uint32_t(b) & kPackedIndex;
+    }
+    return kNone;
+  }
   uint32_t h = cell_hash(x, y, z) & tmask;
   for (uint32_t p = 0; p <= tmask; ++p, h = (h + 1) & tmask) {
     const uint4 b = tab[h];
