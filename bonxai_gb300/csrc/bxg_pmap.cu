@@ -463,11 +463,18 @@ int scan_cube(bxg_pmap_s* pm, int ox, int oy, int oz, double reach, uint64_t ray
   Q->kin = uint32_t(32 * h + 1);
   const size_t blocks = size_t(Q->S) * Q->S * Q->S;
   if (blocks > pm->cube_blocks) {
-    BXG_CUDA(m, pm->cube_bits.ensure(blocks * 64));
+    pm->cube_blocks = 0;
+    const cudaError_t e = pm->cube_bits.ensure(blocks * 64);
+    if (e == cudaErrorMemoryAllocation) {  // the rays are walked on the tree instead
+      cudaGetLastError();
+      *Q = ScanCube{};
+      return BXG_OK;
+    }
+    BXG_CUDA(m, e);
     BXG_CUDA(m, cudaMemsetAsync(pm->cube_bits.p, 0, pm->cube_bits.cap, m->stream));
-    pm->cube_blocks = blocks;
     BXG_CUDA(m, pm->cube_roots.ensure(kRootFlagWords * 4));
     BXG_CUDA(m, cudaMemsetAsync(pm->cube_roots.p, 0, pm->cube_roots.cap, m->stream));
+    pm->cube_blocks = blocks;
     // the batched tick uses the buffers from another stream
     BXG_CUDA(m, cudaStreamSynchronize(m->stream));
   }
