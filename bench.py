@@ -5,8 +5,8 @@ Workload (default ``multimap``): 64 independent ProbabilisticMaps of uneven
 size, each receiving one insertPointCloud scan per tick -- points per map
 log-uniform in [10k, 500k], drawn from the room and LiDAR generators,
 resolutions cycling 0.02 / 0.05 / 0.1 m, max range 10 m, default Options --
-for 50 ticks (``--steps``). Every tick runs through the batched form (one
-graph-replayed persistent launch for all 64 scans) and through the plain
+for 50 ticks (``--steps``). Every tick runs through the batched form (a
+few launches, replayed as one graph, for all 64 scans) and through the plain
 per-scan path (64 synchronous insertPointCloud calls) on identical inputs; the
 two sets of maps are compared bit-exactly after the run.
 
@@ -21,7 +21,7 @@ Metric: ray-cell updates/s, V / t with V = points + sum of cast ray lengths
 * ``e2e``: the batched ticks from pinned host memory through the C ABI
   (host->device copy of the points and read-back of the counters inside).
 * ``tick_ms_p50`` / ``tick_ms_p99``: latency of one batched tick call.
-* ``roofline``: k_tick, algorithmic bytes per tick over its event-timed
+* ``roofline``: the k_tick_* kernels, algorithmic bytes per tick over its event-timed
   duration, against the measured HBM copy bandwidth.
 * ``cpu_baseline``: the CPU path (the oracle restatement, timed against the
   reference in profiles/cpu_port_vs_ref.md) on all host cores, whole maps
@@ -850,7 +850,7 @@ def multimap_config(args, ws):
 
 
 def mm_traffic():
-    """Per-tick DRAM and L2 figures of k_tick from the committed ncu summary."""
+    """Per-tick DRAM and L2 figures of the k_tick_* kernels from the committed ncu summary."""
     p = ROOT / "profiles" / "k_tick_multimap_traffic.json"
     if p.exists():
         try:
@@ -862,7 +862,7 @@ def mm_traffic():
 
 def run_multimap(args):
     """The 64-map uneven workload: every tick, one insertPointCloud scan per
-    map, through the batched form (one graph-replayed persistent launch for
+    map, through the batched form (a few launches, replayed as one graph, for
     all maps) and through the plain per-scan path (one synchronous
     insertPointCloud call per map) on identical inputs; the maps of the two
     paths are compared bit-exactly after the run. Under torchrun each rank
@@ -1000,7 +1000,7 @@ def run_multimap(args):
     if rank != 0:
         dist.destroy_process_group()
         return 0
-    # roofline of k_tick: algorithmic bytes of the timed ticks over their
+    # roofline of the k_tick_* kernels: algorithmic bytes of the timed ticks over their
     # event-timed device duration
     pk, pkind = peaks()
     tick_bytes = (12 * alg["points"] + RAY_LIST_BYTES * alg["rays"] +
@@ -1009,7 +1009,7 @@ def run_multimap(args):
     tick_ms = float(np.mean(dev_ticks))
     ach = tick_bytes / (tick_ms / 1e3) / 1e9
     tr = mm_traffic() or {}
-    roofline = {"kernel": "k_tick (one launch per tick)", "bound": "hbm", "achieved": ach,
+    roofline = {"kernel": "k_tick_* (one graph launch per tick)", "bound": "hbm", "achieved": ach,
                 "peak": pk, "unit": "GB/s", "frac": ach / pk, "peak_kind": pkind,
                 "traffic": tr.get("dram_bytes_per_tick"),
                 "algorithmic_bytes_per_launch": tick_bytes, "launch_ms": tick_ms,

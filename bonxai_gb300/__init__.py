@@ -621,7 +621,7 @@ class ProbabilisticMap(_Handle):
 
 class Batch(_Handle):
     """One insertPointCloud per map for many maps per call, in a few
-    graph-replayed launch (bxg_batch_insert_f32)."""
+    launches replayed as one graph (bxg_batch_insert_f32)."""
     _destroy = "bxg_batch_destroy"
 
     def __init__(self, config: Config | None = None):
