@@ -249,6 +249,8 @@ struct bxg_pmap_s {
   size_t cube_blocks = 0;
   bxg::DevBuf cube_roots, ray_segs, ray_tails;
   bool has_segs = false;  // the ray list's segments are in ray_segs, long rays in ray_tails
+  // the origin cell that the ray list's segments, its long rays and dir_reach are of
+  int list_origin[3] = {0, 0, 0};
   cudaEvent_t ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
   ~bxg_pmap_s() {
     for (auto& e : ev)

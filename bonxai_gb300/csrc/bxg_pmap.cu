@@ -520,6 +520,13 @@ RayKernel ray_kernel(uint32_t rpw, bool u2) {
 int launch_rays(bxg_pmap_s* pm, int ox, int oy, int oz) {
   MapCore* m = &pm->core;
   if (!pm->cast_ub) return BXG_OK;
+  // rays left by a scan that failed, now cast from another origin: how far they reach, and
+  // where they would be cut into segments, is not known
+  const int* lo = pm->list_origin;
+  if (lo[0] != ox || lo[1] != oy || lo[2] != oz) {
+    pm->has_segs = false;
+    pm->dir_reach = 0.0;
+  }
   {
     // two-phase form: mark the rays' cells, then apply per leaf
     ScanCube Q;
@@ -720,6 +727,7 @@ int insert_impl(bxg_pmap m_, const PT* xyz, size_t stride, size_t n, const PT* o
     // rays of this scan end within max_range of the origin (hits are closer);
     // rays queued by earlier add batches may not: no directory then
     pm->dir_reach = pm->cast_ub == 0 ? max_range : 0.0;
+    std::copy(o, o + 3, pm->list_origin);
     // the winners cut the rays of a scan that starts its list into segments
     ScanCube cube{};
     if (pm->cast_ub == 0) {
