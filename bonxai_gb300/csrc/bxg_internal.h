@@ -248,8 +248,10 @@ struct bxg_pmap_s {
   bxg::DevBuf cube_bits;
   size_t cube_blocks = 0;
   bxg::DevBuf cube_roots, ray_segs, ray_tails;
-  bool has_segs = false;  // the ray list's segments are in ray_segs, long rays in ray_tails
-  // the origin cell that the ray list's segments, its long rays and dir_reach are of
+  // the cube that the winners of the ray list knew (no bits: none, the list holds rays of
+  // addHitPoint/addMissPoint batches), whose segments are in ray_segs and long rays in
+  // ray_tails; and the origin cell that it and dir_reach are of
+  bxg::ScanCube list_cube{};
   int list_origin[3] = {0, 0, 0};
   cudaEvent_t ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
   ~bxg_pmap_s() {
@@ -260,7 +262,7 @@ struct bxg_pmap_s {
 
 namespace bxg {
 // The cube of a scan's ray phase from origin cell (ox, oy, oz) whose rays end
-// within `reach` (world units) of the origin; with `reach` unknown (0), infinite or above the
+// within `reach` (world units) of the origin; with `reach` infinite or above the
 // size limit, Q->open is set and the cube holds the rays' first Q->kin
 // cells. *ok = false when the scan cannot use one (other node sizes, non-finite
 // points kept, single pass asked for). rays: room for their segments (0: none).

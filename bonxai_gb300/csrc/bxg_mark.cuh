@@ -131,7 +131,7 @@ struct ScanCube {
   uint32_t* bits;   // S^3 leaf blocks of 16 words, x fastest; zero between scans
   uint32_t* roots;  // one bit per root (SR^3), set by the segments
   uint32_t* segs;   // segments: ray << 8 | number; nullptr: rays are walked whole
-  uint32_t* tails;  // rays longer than kin; nullptr: not listed
+  uint32_t* tails;  // rays longer than kin; nullptr: there are none
   int x0, y0, z0;   // lowest cell (multiples of 32)
   uint32_t S, SR;   // leaves, roots per side
   uint32_t kin;     // cells k < kin of every ray lie in the cube
@@ -727,21 +727,19 @@ __device__ __forceinline__ void endpoint_enter(const DMap& M, int4& e, uint32_t 
 // chain of dependent loads, about 4 us a step, and the rays that go far are few
 // (29 k points at 0.05 m with returns to 100 m: 16 us; with eight rays per warp and
 // pieces of 256 cells 125 us; the whole scan walked by k_rays 330 us, against 17
-// for k_mark, 25 for k_apply_rays and this). Without a list of them (rays queued
-// by addHitPoint/addMissPoint) all rays are looked at.
+// for k_mark, 25 for k_apply_rays and this).
 constexpr uint32_t kTailPieces = 32;
 __device__ __forceinline__ void tail_rays(const DMap& M, const ScanCube& Q,
                                           const int4* __restrict__ cast, uint32_t cast_cap,
                                           uint64_t warp, uint64_t n_warps, int ox, int oy, int oz,
                                           int32_t u, int32_t miss, int32_t cmin,
                                           uint32_t& visited, uint32_t& updated) {
-  const uint32_t n = min(ld_volatile(M.ctr + (Q.tails ? C_TAILS : C_CAST)), cast_cap);
+  const uint32_t n = min(ld_volatile(M.ctr + C_TAILS), cast_cap);
   const unsigned lane = threadIdx.x & 31;
   for (uint64_t t = warp; t < uint64_t(n) * kTailPieces; t += n_warps) {
     const uint32_t i = uint32_t(t / kTailPieces), j = uint32_t(t % kTailPieces);
-    const int4 e = cast[Q.tails ? Q.tails[i] : i];
+    const int4 e = cast[Q.tails[i]];
     const uint32_t m = chebyshev(ox, oy, oz, e.x, e.y, e.z);
-    if (m <= Q.kin) continue;
     if (m >= kMaxRayCells) {
       if (lane == 0) set_err(M, ERR_RAY_TOO_LONG);
       continue;

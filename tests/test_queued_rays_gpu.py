@@ -1,0 +1,63 @@
+"""Rays queued by addHitPoint/addMissPoint: updateFreeCells, and a scan over them, walk them on
+the tree as a map of the single-pass form does, for its time and without scratch memory."""
+import time
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def directions(rng, n):
+    v = rng.normal(size=(n, 3))
+    return v / np.linalg.norm(v, axis=1, keepdims=True)
+
+
+def queue_and_update(m, pts, origin):
+    torch.cuda.synchronize()
+    t = time.perf_counter()
+    m.add_hit_points(pts)
+    m.update_free_cells(origin)
+    return time.perf_counter() - t
+
+
+@pytest.mark.parametrize("res,n,far", [(0.1, 10000, 10.0), (0.05, 20000, 20.0)])
+def test_no_slower_than_the_single_pass_form(gpu, res, n, far):
+    rng = np.random.default_rng(4)
+    batches = [torch.from_numpy(directions(rng, n) * rng.uniform(2, far, (n, 1))).cuda()
+               for _ in range(4)]
+    maps = [gpu.ProbabilisticMap(res, gpu.Config(flags=f))
+            for f in (0, gpu.FLAG_RAYS_SINGLE_PASS)]
+    took = [[], []]
+    for k in range(20):
+        for m, t in zip(maps, took):
+            t.append(queue_and_update(m, batches[k % 4], np.array([0.3 * (k % 4), 0.1, 0.2])))
+    # the same kernels; two runs of one of them differ by a tenth
+    assert np.median(took[0][6:]) < 1.3 * np.median(took[1][6:])
+    assert all(np.array_equal(a, b) for a, b in zip(maps[0].dump(), maps[1].dump()))
+
+
+def test_cost_does_not_grow_from_call_to_call(gpu):
+    rng = np.random.default_rng(5)
+    one = torch.tensor([[0.55, 0.0, 0.0]], dtype=torch.float64, device="cuda")
+    m = gpu.ProbabilisticMap(0.1)
+    origin = np.zeros(3)
+    new = np.median([queue_and_update(m, one, origin) for _ in range(30)][6:])
+    for _ in range(4):  # rays in all directions
+        m.add_hit_points(directions(rng, 40000) * rng.uniform(5, 50, (40000, 1)))
+        m.update_free_cells(origin)
+    used = np.median([queue_and_update(m, one, origin) for _ in range(30)][6:])
+    assert used < 1.5 * new
+
+
+def test_no_scratch_bitmap(gpu):
+    m = gpu.ProbabilisticMap(0.1)
+    m.insert_point_cloud(np.ones((10, 3), np.float32), np.zeros(3, np.float32), 2.0)
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    m.add_hit_points(np.ones((1, 3)))
+    m.update_free_cells(np.zeros(3))
+    m.add_miss_points(np.ones((1, 3)))
+    m.insert_point_cloud(np.ones((10, 3), np.float32), np.zeros(3, np.float32), 2.0)
+    assert before - torch.cuda.mem_get_info()[0] < 16 << 20
