@@ -207,11 +207,13 @@ __device__ __forceinline__ uint32_t cell_hash(int x, int y, int z) {
 // ---------------------------------------------------------------------------
 // slot allocation
 // ---------------------------------------------------------------------------
-// A counter step for each of the threads that are here together, as one atomic per warp:
-// thousands of new nodes take their slots from one word, and its atomics with a
-// result come out of L2 one after the other.
+// A counter step for each of the threads that are here together, as one atomic per counter
+// and warp (the lanes of a tick's warp may belong to different maps): thousands of new nodes
+// take their slots from one word, and its atomics with a result come out of L2 one after
+// the other.
 __device__ __forceinline__ uint32_t counter_step(uint32_t* c) {
-  const unsigned here = __activemask();
+  const unsigned here =
+      __match_any_sync(__activemask(), reinterpret_cast<unsigned long long>(c));
   const unsigned lane = threadIdx.x & 31;
   const int lead = __ffs(static_cast<int>(here)) - 1;
   uint32_t base = 0;
