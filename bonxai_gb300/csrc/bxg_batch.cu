@@ -671,7 +671,7 @@ cudaError_t enqueue_tick(bxg_batch b, size_t param_bytes, size_t smem, bool mark
 namespace bxg {
 int batch_insert(bxg_batch b, const bxg_pmap* maps, size_t n_scans, const float* xyz,
                  const float* const* parts, const uint64_t* offsets, const float* origins,
-                 const double* max_ranges, uint64_t* ray_cells) {
+                 const double* max_ranges, uint64_t* ray_cells, size_t cube_room) {
   if (!b) return BXG_ERR_INVALID_ARG;
   if (!n_scans) return BXG_OK;
   if (!maps || !offsets || !origins || !max_ranges)
@@ -785,6 +785,11 @@ int batch_insert(bxg_batch b, const bxg_pmap* maps, size_t n_scans, const float*
   for (size_t s = 0; s < n_scans && mark; s++) {
     TickScan& S = b->h_scans[s];
     bool ok = false;
+    if (open_reach(&maps[s]->core, S.max_range) && maps[s]->cube_blocks < kOpenCubeBlocks) {
+      mark = cube_room >= kOpenCubeBytes;
+      if (!mark) break;
+      cube_room -= kOpenCubeBytes;
+    }
     const int st = scan_cube(maps[s], S.ox, S.oy, S.oz, S.max_range, 0, &S.Q, &ok);
     if (st) return bfail(b, st, maps[s]->core.err);
     mark = ok;
@@ -992,7 +997,8 @@ int bxg_batch_insert_f32(bxg_batch b, const bxg_pmap* maps, size_t n_scans, cons
   if (!b) return BXG_ERR_INVALID_ARG;
   if (!n_scans) return BXG_OK;
   if (!xyz) return bfail(b, BXG_ERR_INVALID_ARG, "null argument");
-  return batch_insert(b, maps, n_scans, xyz, nullptr, offsets, origins, max_ranges, ray_cells);
+  return batch_insert(b, maps, n_scans, xyz, nullptr, offsets, origins, max_ranges, ray_cells,
+                      SIZE_MAX);
 }
 int bxg_batch_phase_ms(bxg_batch b, double out[6]) {
   if (!b || !out) return BXG_ERR_INVALID_ARG;

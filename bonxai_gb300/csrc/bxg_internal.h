@@ -28,6 +28,15 @@ struct DevBuf {
     if (e == cudaSuccess) cap = want;
     return e;
   }
+  // Like ensure, but not rounded up.
+  cudaError_t ensure_exact(size_t bytes) {
+    if (bytes <= cap) return cudaSuccess;
+    release();
+    const cudaError_t e = cudaMalloc(&p, bytes);
+    if (e == cudaSuccess) cap = bytes;
+    else p = nullptr;
+    return e;
+  }
   // Like ensure, but keeps the first `keep` bytes of the old content.
   cudaError_t ensure_keep(size_t bytes, size_t keep, cudaStream_t s) {
     if (bytes <= cap) return cudaSuccess;
@@ -269,6 +278,17 @@ namespace bxg {
 // Buffers grow here (cudaMalloc, zeroed).
 int scan_cube(bxg_pmap_s* pm, int ox, int oy, int oz, double reach, uint64_t rays, ScanCube* Q,
               bool* ok);
+// The bitmap of an open cube, 147 MB, is memory that such a scan can do without (its rays are
+// walked on the tree then). It counts against the map's budget, behind the pools: it is
+// made, and held, while both fit.
+constexpr size_t kOpenCubeBlocks =
+    size_t(4 * (2 * kOpenCubeHalf + 1)) * (4 * (2 * kOpenCubeHalf + 1)) * (4 * (2 * kOpenCubeHalf + 1));
+constexpr size_t kOpenCubeBytes = kOpenCubeBlocks * 64;
+// A scan of this reach takes an open cube.
+bool open_reach(const MapCore* m, double reach);
+// Bytes of an open cube's bitmap that the map holds.
+size_t open_cube_held(const bxg_pmap_s* pm);
+void drop_open_cube(bxg_pmap_s* pm);
 // Sets up the ray walk's leaf directory of a scan (bxg_pmap.cu).
 int leaf_dir_for_scan(bxg_pmap_s* pm, int ox, int oy, int oz, LeafDir* D, size_t max_words);
 // Completes a scan whose endpoints were listed (and possibly applied) by a
@@ -277,10 +297,10 @@ int leaf_dir_for_scan(bxg_pmap_s* pm, int ox, int oy, int oz, LeafDir* D, size_t
 int pmap_complete_scan(bxg_pmap_s* pm, const int4* d_cast, const uint32_t* d_count,
                        uint32_t cap, int ox, int oy, int oz, int32_t u);
 // bxg_batch_insert_f32, with the points of scan s either at xyz + 3 offsets[s] or, with
-// parts, in host memory at parts[s].
+// parts, in host memory at parts[s]. New bitmaps of open cubes take at most cube_room bytes.
 int batch_insert(bxg_batch b, const bxg_pmap* maps, size_t n_scans, const float* xyz,
                  const float* const* parts, const uint64_t* offsets, const float* origins,
-                 const double* max_ranges, uint64_t* ray_cells);
+                 const double* max_ranges, uint64_t* ray_cells, size_t cube_room);
 // Grows the map's pools so that the next scan has at least `leaves` free leaf
 // slots and the root hash stays under its load factor.
 int core_reserve(MapCore* m, size_t leaves, size_t inners);

@@ -442,6 +442,24 @@ int leaf_dir_for_scan(bxg_pmap_s* pm, int ox, int oy, int oz, LeafDir* D, size_t
 }  // namespace bxg
 
 namespace bxg {
+// Ray ends lie within this many cells of the origin cell (the floor of the origin and of
+// the end each move a cell by less than one).
+static double reach_cells(const MapCore* m, double reach) {
+  return std::ceil(reach * m->inv_res) + 2.0;
+}
+bool open_reach(const MapCore* m, double reach) {
+  return !(reach_cells(m, reach) <= 32.0 * kMaxCubeHalf);
+}
+size_t open_cube_held(const bxg_pmap_s* pm) {
+  return pm->cube_bits.cap == kOpenCubeBytes ? kOpenCubeBytes : 0;
+}
+void drop_open_cube(bxg_pmap_s* pm) {
+  if (!open_cube_held(pm)) return;
+  pm->cube_bits.release();
+  pm->cube_blocks = 0;
+  pm->list_cube = ScanCube{};
+}
+
 int scan_cube(bxg_pmap_s* pm, int ox, int oy, int oz, double reach, uint64_t rays, ScanCube* Q,
               bool* ok) {
   MapCore* m = &pm->core;
@@ -450,14 +468,17 @@ int scan_cube(bxg_pmap_s* pm, int ox, int oy, int oz, double reach, uint64_t ray
   if (m->dm.lb != 3 || m->dm.ib != 2 || m->dm.esz != 4 ||
       (m->flags & (BXG_FLAG_KEEP_NONFINITE | BXG_FLAG_RAYS_SINGLE_PASS)) || !(reach > 0))
     return BXG_OK;
-  // Ray ends lie within ceil(reach / res) + 2 cells of the origin cell (the
-  // floor of the origin and of the end each move a cell by less than one).
-  const double cells = std::ceil(reach * m->inv_res) + 2.0;
   int h = kOpenCubeHalf;
-  if (cells <= 32.0 * kMaxCubeHalf)
-    h = std::max(1, (int(cells) + 31) / 32);
-  else
+  if (open_reach(m, reach)) {
     Q->open = 1;
+    if (core_mem_usage(m) + kOpenCubeBytes > m->budget) {
+      drop_open_cube(pm);
+      *Q = ScanCube{};
+      return BXG_OK;
+    }
+  } else {
+    h = std::max(1, (int(reach_cells(m, reach)) + 31) / 32);
+  }
   Q->SR = uint32_t(2 * h + 1);
   Q->S = 4 * Q->SR;
   // cells k <= 32 h of a ray lie within h roots of the origin's
@@ -465,7 +486,8 @@ int scan_cube(bxg_pmap_s* pm, int ox, int oy, int oz, double reach, uint64_t ray
   const size_t blocks = size_t(Q->S) * Q->S * Q->S;
   if (blocks > pm->cube_blocks) {
     pm->cube_blocks = 0;
-    const cudaError_t e = pm->cube_bits.ensure(blocks * 64);
+    const cudaError_t e = Q->open ? pm->cube_bits.ensure_exact(blocks * 64)
+                                  : pm->cube_bits.ensure(blocks * 64);
     if (e == cudaErrorMemoryAllocation) {  // the rays are walked on the tree instead
       cudaGetLastError();
       *Q = ScanCube{};

@@ -432,6 +432,7 @@ void worker_loop(bxg_server_s* s) {
       if (mt.mid->kind != K_CLEAR) continue;
       bxg_pmap m = s->maps[mt.map];
       m->cast_ub = 0;
+      if (mt.mid->mode) drop_open_cube(m);
       mt.mid->status = mt.mid->mode ? core_release_pools(&m->core) : core_clear(&m->core);
       mt.mid->t_start = t0;
     }
@@ -463,6 +464,13 @@ void worker_loop(bxg_server_s* s) {
       }
     }
     if (!admit.empty()) {
+      // what the pools leave of the budget is for bitmaps of scans without a range limit
+      size_t held = 0;
+      for (bxg_pmap m : s->maps) held += open_cube_held(m);
+      if (used + held > s->budget) {
+        for (bxg_pmap m : s->maps) drop_open_cube(m);
+        held = 0;
+      }
       std::vector<bxg_pmap> ms;
       std::vector<uint64_t> off(1, 0);
       std::vector<float> org;
@@ -478,7 +486,7 @@ void worker_loop(bxg_server_s* s) {
       for (MapTick* mt : admit) parts.push_back(mt->mid->pts.data());
       std::vector<uint64_t> rc(admit.size(), 0);
       st = batch_insert(s->batch, ms.data(), ms.size(), nullptr, parts.data(), off.data(),
-                        org.data(), mr.data(), rc.data());
+                        org.data(), mr.data(), rc.data(), s->budget - used - held);
       for (size_t k = 0; k < admit.size(); k++) {
         admit[k]->mid->status = st;
         admit[k]->mid->ray_cells = rc[k];

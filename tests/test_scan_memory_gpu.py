@@ -1,0 +1,84 @@
+"""Scratch memory that a scan can do without (the bitmap of a scan whose rays have no range
+limit) is held within the map's budget; without it the scan gives the same map."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+MB = 1 << 20
+INF = float("inf")
+
+
+def clouds(seed, k, n=4000, far=30.0):
+    rng = np.random.default_rng(seed)
+    out = []
+    for _ in range(k):
+        d = rng.normal(size=(n, 3))
+        d /= np.linalg.norm(d, axis=1, keepdims=True)
+        out.append((d * rng.uniform(1, far, (n, 1))).astype(np.float32))
+    return out
+
+
+def free_bytes():
+    torch.cuda.synchronize()
+    return torch.cuda.mem_get_info()[0]
+
+
+def same(gmap, omap):
+    assert all(np.array_equal(a, b) for a, b in zip(gmap.dump(), omap.dump()))
+
+
+# 14 k leaves at most, 30 MB: the bitmap of 147 MB fits behind the pools, or never, or only
+# until the pools have grown
+@pytest.mark.parametrize("budget,leaves", [(0, 16384), (100 * MB, 16384), (170 * MB, 0)])
+def test_scans_without_a_range_limit(gpu, port, budget, leaves):
+    scans = clouds(1, 6, 1000, 12.0)
+    m = gpu.ProbabilisticMap(0.1, gpu.Config(pool_budget_bytes=budget, initial_leaves=leaves))
+    o = port.pmap(0.1)
+    for k, p in enumerate(scans):
+        m.insert_point_cloud(p[:200], np.zeros(3, np.float32), 2.0)  # buffers of the staging
+        o.insert(p[:200], np.zeros(3, np.float32), 2.0)
+        before = free_bytes()
+        assert m.insert_point_cloud(p, np.zeros(3, np.float32), INF) == \
+            o.insert(p, np.zeros(3, np.float32), INF)
+        if k == 0 and leaves:  # no pool grows: the bitmap, and some hundred bytes a point
+            assert before - free_bytes() < (8 * MB if budget else 155 * MB)
+        if budget:
+            assert m.mem_usage() <= budget
+    same(m, o)
+
+
+def test_a_tick_without_a_range_limit(gpu, port):
+    maps = [gpu.ProbabilisticMap(0.1, gpu.Config(pool_budget_bytes=b))
+            for b in (0, 100 * MB, 0)]
+    orc = [port.pmap(0.1) for _ in maps]
+    b = gpu.Batch()
+    for k in range(3):
+        scans = clouds(10 + k, len(maps), 2000, 12.0)
+        off = np.arange(len(maps) + 1) * 2000
+        got = b.insert(maps, np.concatenate(scans), off, np.zeros((len(maps), 3)),
+                       [INF, INF, 10.0])
+        assert [int(v) for v in got] == [o.insert(p, np.zeros(3, np.float32), r)
+                                         for o, p, r in zip(orc, scans, (INF, INF, 10.0))]
+    for m, o in zip(maps, orc):
+        same(m, o)
+
+
+def test_a_server_without_a_range_limit(gpu, port):
+    """The bitmaps of a server's maps are within its budget, behind the pools."""
+    n, budget = 6, 400 * MB
+    before = free_bytes()
+    s = gpu.Server([0.2] * n, gpu.ServerConfig(pool_budget_bytes=budget))
+    orc = [port.pmap(0.2) for _ in range(n)]
+    for k in range(4):
+        scans = clouds(20 + k, n, 1000, 20.0)
+        tickets = [s.insert(i, p, np.zeros(3, np.float32), INF) for i, p in enumerate(scans)]
+        for t, p, o in zip(tickets, scans, orc):
+            assert s.wait_insert(t)["ray_cells"] == o.insert(p, np.zeros(3, np.float32), INF)
+    s.drain()
+    # beside the budget: the lists and tables of ticks of 6,000 points
+    assert before - free_bytes() < budget + 64 * MB
+    for i, o in enumerate(orc):
+        assert all(np.array_equal(a, b) for a, b in zip(s.map_dump(i), o.dump()))
+    s.close()
