@@ -121,6 +121,7 @@ _SIGS = {
     "bxg_pmap_stream": (_vp, [_vp]),
     "bxg_pmap_grid": (_vp, [_vp]),
     "bxg_debug_hold_leaf": (_int, [_vp, _vp]),
+    "bxg_debug_alloc_limit": (_int, [_sz]),
     "bxg_pmap_last_query_ms": (_int, [_vp, _vp]),
     "bxg_pmap_add_points": (_int, [_vp, _vp, _vp, _sz]),
     "bxg_grid_store_if_on": (_int, [_vp, _vp, _vp, _sz]),

@@ -808,9 +808,14 @@ int batch_insert(bxg_batch b, const bxg_pmap* maps, size_t n_scans, const float*
     if (has_segs[s]) seg_room += need;
   }
   if (mark) {
-    BB_CUDA(b, grow(b->segs, seg_room * 4 + 16));
-    BB_CUDA(b, grow(b->roots, root_room * 4 + 16));
-    if (tail) BB_CUDA(b, grow(b->tails, total * 4 + 16));
+    cudaError_t e = grow(b->segs, seg_room * 4 + 16);
+    if (e == cudaSuccess) e = grow(b->roots, root_room * 4 + 16);
+    if (e == cudaSuccess && tail) e = grow(b->tails, total * 4 + 16);
+    mark = e != cudaErrorMemoryAllocation;  // else the rays are walked on the tree
+    if (mark) BB_CUDA(b, e);
+    cudaGetLastError();
+  }
+  if (mark) {
     A.roots = b->roots.as<uint32_t>();
     for (size_t s = 0; s < n_scans; s++) {
       TickScan& S = b->h_scans[s];

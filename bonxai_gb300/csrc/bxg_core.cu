@@ -648,6 +648,11 @@ const char* bxg_status_string(int s) {
 
 int bxg_version(void) { return 100; }
 
+int bxg_debug_alloc_limit(size_t bytes) {
+  bxg::DevBuf::limit = bytes;
+  return BXG_OK;
+}
+
 const char* bxg_last_error(const void* handle) {
   if (!handle) return bxg::g_create_error.c_str();
   return bxg::core_of_handle(handle)->err.c_str();

@@ -17,24 +17,25 @@ namespace bxg {
 struct DevBuf {
   void* p = nullptr;
   size_t cap = 0;
+  // Test hook (bxg_debug_alloc_limit): this host thread's larger requests fail as they do on
+  // a device without memory.
+  static inline thread_local size_t limit = SIZE_MAX;
+  static cudaError_t alloc(void** q, size_t bytes) {
+    *q = nullptr;
+    return bytes <= limit ? cudaMalloc(q, bytes) : cudaErrorMemoryAllocation;
+  }
   cudaError_t ensure(size_t bytes) {
     if (bytes <= cap) return cudaSuccess;
     size_t want = cap ? cap : 4096;
     while (want < bytes) want *= 2;
-    if (p) cudaFree(p);
-    p = nullptr;
-    cap = 0;
-    cudaError_t e = cudaMalloc(&p, want);
-    if (e == cudaSuccess) cap = want;
-    return e;
+    return ensure_exact(want);
   }
   // Like ensure, but not rounded up.
   cudaError_t ensure_exact(size_t bytes) {
     if (bytes <= cap) return cudaSuccess;
     release();
-    const cudaError_t e = cudaMalloc(&p, bytes);
+    const cudaError_t e = alloc(&p, bytes);
     if (e == cudaSuccess) cap = bytes;
-    else p = nullptr;
     return e;
   }
   // Like ensure, but keeps the first `keep` bytes of the old content.
@@ -43,7 +44,7 @@ struct DevBuf {
     size_t want = cap ? cap : 4096;
     while (want < bytes) want *= 2;
     void* np = nullptr;
-    cudaError_t e = cudaMalloc(&np, want);
+    cudaError_t e = alloc(&np, want);
     if (e != cudaSuccess) return e;
     if (p && keep) {
       e = cudaMemcpyAsync(np, p, keep < cap ? keep : cap, cudaMemcpyDeviceToDevice, s);
@@ -274,8 +275,8 @@ namespace bxg {
 // within `reach` (world units) of the origin; with `reach` infinite or above the
 // size limit, Q->open is set and the cube holds the rays' first Q->kin
 // cells. *ok = false when the scan cannot use one (other node sizes, non-finite
-// points kept, single pass asked for). rays: room for their segments (0: none).
-// Buffers grow here (cudaMalloc, zeroed).
+// points kept, single pass asked for, no memory for it). rays: room for their
+// segments (0: none). Buffers grow here (cudaMalloc, zeroed).
 int scan_cube(bxg_pmap_s* pm, int ox, int oy, int oz, double reach, uint64_t rays, ScanCube* Q,
               bool* ok);
 // The bitmap of an open cube, 147 MB, is memory that such a scan can do without (its rays are

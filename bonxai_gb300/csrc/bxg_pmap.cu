@@ -395,7 +395,7 @@ namespace bxg {
 // for several scans, takes the next epoch. The whole buffer is cleared when
 // the 4-bit epoch wraps, so a word of another epoch is always empty. *D stays
 // empty (the walk probes the root hash for every leaf run) when the cube would
-// exceed max_words words or leaf slots do not fit in 28 bits.
+// exceed max_words words, when there is no memory for it, or leaf slots do not fit in 28 bits.
 int leaf_dir_for_scan(bxg_pmap_s* pm, int ox, int oy, int oz, LeafDir* D, size_t max_words) {
   MapCore* m = &pm->core;
   *D = LeafDir{};
@@ -416,7 +416,13 @@ int leaf_dir_for_scan(bxg_pmap_s* pm, int ox, int oy, int oz, LeafDir* D, size_t
     if (words_of(h) > max_words) return BXG_OK;
     const size_t words = words_of(h);
     if (m->s_dir.cap < words * 4) {
-      BXG_CUDA(m, m->s_dir.ensure(words * 4));
+      pm->dir_live = false;
+      const cudaError_t e = m->s_dir.ensure(words * 4);
+      if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        return BXG_OK;
+      }
+      BXG_CUDA(m, e);
       BXG_CUDA(m, cudaMemsetAsync(m->s_dir.p, 0, m->s_dir.cap, m->stream));
       pm->dir_epoch = 0;
     }
@@ -484,18 +490,24 @@ int scan_cube(bxg_pmap_s* pm, int ox, int oy, int oz, double reach, uint64_t ray
   // cells k <= 32 h of a ray lie within h roots of the origin's
   Q->kin = uint32_t(32 * h + 1);
   const size_t blocks = size_t(Q->S) * Q->S * Q->S;
-  if (blocks > pm->cube_blocks) {
-    pm->cube_blocks = 0;
-    const cudaError_t e = Q->open ? pm->cube_bits.ensure_exact(blocks * 64)
-                                  : pm->cube_bits.ensure(blocks * 64);
-    if (e == cudaErrorMemoryAllocation) {  // the rays are walked on the tree instead
+  // Without memory for one of the buffers the rays are walked on the tree.
+  auto grow = [&](DevBuf& b, size_t bytes, bool exact, bool* got) -> int {
+    const cudaError_t e = exact ? b.ensure_exact(bytes) : b.ensure(bytes);
+    *got = e == cudaSuccess;
+    if (e != cudaSuccess && e != cudaErrorMemoryAllocation) BXG_CUDA(m, e);
+    if (!*got) {
       cudaGetLastError();
       *Q = ScanCube{};
-      return BXG_OK;
     }
-    BXG_CUDA(m, e);
+    return BXG_OK;
+  };
+  bool got = true;
+  if (blocks > pm->cube_blocks) {
+    pm->cube_blocks = 0;
+    int st = grow(pm->cube_bits, blocks * 64, Q->open != 0, &got);
+    if (!st && got) st = grow(pm->cube_roots, kRootFlagWords * 4, false, &got);
+    if (st || !got) return st;
     BXG_CUDA(m, cudaMemsetAsync(pm->cube_bits.p, 0, pm->cube_bits.cap, m->stream));
-    BXG_CUDA(m, pm->cube_roots.ensure(kRootFlagWords * 4));
     BXG_CUDA(m, cudaMemsetAsync(pm->cube_roots.p, 0, pm->cube_roots.cap, m->stream));
     pm->cube_blocks = blocks;
     // the batched tick uses the buffers from another stream
@@ -504,11 +516,13 @@ int scan_cube(bxg_pmap_s* pm, int ox, int oy, int oz, double reach, uint64_t ray
   // a segment is a ray's position (24 bits) and a number (8 bits)
   const uint64_t segs = rays * max_segments(*Q);
   if (rays && rays <= (1u << 24) && segs <= (1u << 28)) {
-    BXG_CUDA(m, pm->ray_segs.ensure(segs * 4));
+    const int st = grow(pm->ray_segs, segs * 4, false, &got);
+    if (st || !got) return st;
     Q->segs = pm->ray_segs.as<uint32_t>();
   }
   if (rays && Q->open) {
-    BXG_CUDA(m, pm->ray_tails.ensure(rays * 4));
+    const int st = grow(pm->ray_tails, rays * 4, false, &got);
+    if (st || !got) return st;
     Q->tails = pm->ray_tails.as<uint32_t>();
   }
   Q->bits = pm->cube_bits.as<uint32_t>();

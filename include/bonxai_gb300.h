@@ -211,6 +211,9 @@ int bxg_grid_read_leaf(bxg_grid g, const int32_t xyz[3], uint64_t* inner_mask,
  * the mark. For tests of the bounded waits only. BXG_ERR_INVALID_ARG if that
  * leaf already exists. */
 int bxg_debug_hold_leaf(bxg_grid g, const int32_t xyz[3]);
+/* Test hook: requests of this host thread's calls for more device memory than this at once
+ * fail as on a device without memory (SIZE_MAX, the default: none does). */
+int bxg_debug_alloc_limit(size_t bytes);
 
 /* Serialize(out, grid) (bonxai_core/include/bonxai/serialization.hpp:77-116):
  * the reference's byte format -- header line

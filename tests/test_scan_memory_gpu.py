@@ -82,3 +82,71 @@ def test_a_server_without_a_range_limit(gpu, port):
     for i, o in enumerate(orc):
         assert all(np.array_equal(a, b) for a, b in zip(s.map_dump(i), o.dump()))
     s.close()
+
+
+@pytest.fixture
+def alloc_limit(gpu):
+    """Sets the largest request for device memory that does not fail."""
+    lib = gpu.load_library()
+    yield lib.bxg_debug_alloc_limit
+    lib.bxg_debug_alloc_limit(2**64 - 1)
+
+
+def sphere(rng, n, radius):
+    """n points in all directions; far ones in a cone, which crosses few leaves."""
+    d = rng.normal(size=(n, 3))
+    if radius > 20:
+        d = d * (0.0, 0.05, 0.05) + (1.0, 0.0, 0.0)
+    return (d / np.linalg.norm(d, axis=1, keepdims=True) * radius).astype(np.float32)
+
+
+# the first scans' buffers are made before the limit: then only the list of segments has to
+# grow, or the bitmap (and what follows it), or the list of rays that leave the cube
+@pytest.mark.parametrize("warm,max_range", [((10.0, 100), 10.0), ((3.0, 100), 10.0),
+                                            ((INF, 100), INF)])
+def test_a_scan_that_finds_no_memory_for_its_lists(gpu, port, alloc_limit, warm, max_range):
+    rng = np.random.default_rng(7)
+    n, zero = 60000, np.zeros(3, np.float32)
+    m = gpu.ProbabilisticMap(0.1, gpu.Config(initial_leaves=1 << 17, initial_inners=1 << 13,
+                                             hash_buckets=1 << 15))
+    o = port.pmap(0.1)
+    big = [sphere(rng, n, 9.0 if np.isfinite(max_range) else 60.0) for _ in range(3)]
+    first = [(sphere(rng, n, 2.0), 2.5), (big[0][:warm[1]], warm[0])]
+    for p, r in first:
+        assert m.insert_point_cloud(p, zero, r) == o.insert(p, zero, r)
+    p = sphere(rng, n, 2.0).astype(np.float64)  # the table of a scan without a bitmap
+    m.add_hit_points(p)
+    o.add_hit(p)
+    assert m.update_free_cells(np.zeros(3)) == o.update_free_cells(np.zeros(3))
+    assert alloc_limit(60000) == 0  # less than four bytes a point
+    for p in big:
+        assert m.insert_point_cloud(p, zero, max_range) == o.insert(p, zero, max_range)
+    alloc_limit(2**64 - 1)
+    for p in big:
+        assert m.insert_point_cloud(p, zero, max_range) == o.insert(p, zero, max_range)
+    same(m, o)
+
+
+@pytest.mark.parametrize("max_range", [10.0, INF])
+def test_a_tick_that_finds_no_memory_for_its_lists(gpu, port, alloc_limit, max_range):
+    rng = np.random.default_rng(8)
+    n, k, zero = 20000, 3, np.zeros((3, 3), np.float32)
+    cfg = gpu.Config(initial_leaves=1 << 17, initial_inners=1 << 13, hash_buckets=1 << 15)
+    maps = [gpu.ProbabilisticMap(0.1, cfg) for _ in range(k)]
+    orc = [port.pmap(0.1) for _ in range(k)]
+    b = gpu.Batch()
+
+    def tick(scans, r):
+        off = np.concatenate([[0], np.cumsum([len(p) for p in scans])])
+        got = b.insert(maps, np.concatenate(scans), off, zero, r)
+        assert [int(v) for v in got] == [w.insert(p, z, r) for w, p, z in zip(orc, scans, zero)]
+
+    tick([sphere(rng, n, 2.0) for _ in maps], 2.5)
+    tick([sphere(rng, 50, 9.0) for _ in maps], max_range)
+    assert alloc_limit(60000) == 0
+    for _ in range(2):
+        tick([sphere(rng, n, 9.0 if np.isfinite(max_range) else 60.0) for _ in maps], max_range)
+    alloc_limit(2**64 - 1)
+    tick([sphere(rng, n, 9.0) for _ in maps], max_range)
+    for m, o in zip(maps, orc):
+        same(m, o)
