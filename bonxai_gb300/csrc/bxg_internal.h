@@ -219,11 +219,12 @@ int run_with_growth(MapCore* m, F&& body) {
 // point: 2k points 10.2, 6.2, 5.3, 4.9 us; 60k room 11.6, 8.9, 8.3, 7.7 us with 17.4, 17.3,
 // 17.6, 19.6 us for k_mark, which clears it; 131k LiDAR 9.1, 7.6, 7.2, 7.2 with 24.9, 25.9,
 // 26.3, 27.6; 64 maps of 10-500 k points 264, 250, 248, 245 us with 55, 110, 219, 440 us to
-// clear. The grid batches' tables are sized by the same rule.
+// clear. The grid batches' tables are sized by the same rule. From 2^30 points it is 2^31
+// entries, more than there are points in the largest batch (2^31 - 2).
 inline uint32_t dedup_entries(uint64_t n) {
   const uint64_t per = n <= (1u << 13) ? 16 : n <= (1u << 16) ? 8 : n <= (1u << 17) ? 4 : 2;
   uint32_t p = 64;
-  while (p < per * n) p <<= 1;
+  while (p < per * n && p < (1u << 31)) p <<= 1;
   return p;
 }
 
