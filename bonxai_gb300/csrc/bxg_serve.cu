@@ -24,7 +24,6 @@
 #include <algorithm>
 #include <chrono>
 #include <condition_variable>
-#include <cstdlib>
 #include <cstring>
 #include <deque>
 #include <mutex>
@@ -32,6 +31,7 @@
 #include <unordered_map>
 #include <vector>
 
+#include "bxg_hostpool.h"
 #include "bxg_internal.h"
 
 namespace bxg {
@@ -83,83 +83,15 @@ using namespace bxg;
 using Clock = std::chrono::steady_clock;
 
 namespace {
-// Page-locked host buffers of the requests' inputs, kept between requests: the client's
-// copy into one touches no new pages, and the worker's copy to the GPU reads it in place.
-// A client only takes a free buffer, else plain memory (page-locking is a call into the
-// driver that may not be made during a stream capture); the worker makes the buffers that were
-// missed, until kMost bytes are held. They are freed with the server.
-class HostPool {
- public:
-  static constexpr size_t kMost = size_t(256) << 20;
-  static constexpr size_t kLeast = size_t(64) << 10;
-  // *cap: the size of a pooled buffer, 0 for plain memory.
-  void* take(size_t bytes, size_t* cap) {
-    size_t c = 0;
-    const int k = class_of(bytes, &c);
-    if (k < kClasses) {
-      std::lock_guard<std::mutex> lk(mu_);
-      if (!free_[k].empty()) {
-        void* p = free_[k].back();
-        free_[k].pop_back();
-        *cap = c;
-        return p;
-      }
-      missed_[k]++;
-    }
-    *cap = 0;
-    return std::malloc(bytes ? bytes : 1);
+void* pinned_alloc(size_t bytes) {
+  void* p = nullptr;
+  if (cudaMallocHost(&p, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
   }
-  void give(void* p, size_t cap) {
-    if (!cap) {
-      std::free(p);
-      return;
-    }
-    size_t c = 0;
-    const int k = class_of(cap, &c);
-    std::lock_guard<std::mutex> lk(mu_);
-    free_[k].push_back(p);
-  }
-  // (worker) Makes a buffer for each request that found none.
-  void refill() {
-    for (int k = 0; k < kClasses; ++k) {
-      const size_t c = kLeast << k;
-      for (;;) {
-        {
-          std::lock_guard<std::mutex> lk(mu_);
-          if (!missed_[k] || held_ + c > kMost) {
-            missed_[k] = 0;
-            break;
-          }
-          missed_[k]--;
-          held_ += c;
-        }
-        void* p = nullptr;
-        if (cudaMallocHost(&p, c) != cudaSuccess) {
-          cudaGetLastError();
-          return;
-        }
-        std::lock_guard<std::mutex> lk(mu_);
-        free_[k].push_back(p);
-      }
-    }
-  }
-  ~HostPool() {
-    for (auto& f : free_)
-      for (void* p : f) cudaFreeHost(p);
-  }
-
- private:
-  static constexpr int kClasses = 13;  // 64 KB .. 256 MB
-  static int class_of(size_t bytes, size_t* c) {
-    int k = 0;
-    for (*c = kLeast; *c < bytes; *c <<= 1) ++k;
-    return k;
-  }
-  std::mutex mu_;
-  std::vector<void*> free_[kClasses];
-  size_t missed_[kClasses] = {0};
-  size_t held_ = 0;
-};
+  return p;
+}
+void pinned_free(void* p) { cudaFreeHost(p); }
 
 // An input array in a buffer of the pool.
 template <class T>
@@ -217,7 +149,7 @@ struct Request {
 }  // namespace
 
 struct bxg_server_s {
-  HostPool pool;  // outlives the requests, which the destructor below deletes
+  HostPool pool{pinned_alloc, pinned_free};  // outlives the requests, which the destructor below deletes
   int device = 0;
   std::vector<bxg_pmap> maps;
   bxg_batch batch = nullptr;
@@ -668,6 +600,7 @@ int bxg_server_create(bxg_server* out, const double* resolutions, size_t n_maps,
     delete s;
     return st;
   }
+  s->pool.start();
   s->fifo.resize(n_maps);
   s->worker = std::thread(worker_loop, s);
   *out = s;
