@@ -217,23 +217,24 @@ __global__ void k_get_values(const __grid_constant__ DMap M, const int32_t* __re
   const int x = xyz[3 * i], y = xyz[3 * i + 1], z = xyz[3 * i + 2];
   const uint32_t lf = leaf_of(M, x, y, z, create != 0);
   bool on = false;
-  uint32_t ci = 0;
-  uint8_t* d = out_vals + static_cast<size_t>(i) * ESZ;
+  unsigned long long v = 0;  // the value's bytes
+  uint8_t* const vp = reinterpret_cast<uint8_t*>(&v);
   if (lf != kNone) {
-    ci = leaf_index(M, x, y, z);
-    // an off cell holds T{}: its content is the answer whatever the mask says, and
-    // neither load waits for the other
+    const uint32_t ci = leaf_index(M, x, y, z);
+    // the value is on its way while the mask word is
     if (ESZ > 0 && out_vals)
-      copy_val<ESZ>(d, M.ldata + (static_cast<size_t>(lf) * M.lsize + ci) * ESZ);
+      copy_val<ESZ>(vp, M.ldata + (static_cast<size_t>(lf) * M.lsize + ci) * ESZ);
     if (create) {
       cell_or_on(M, lf, ci);
       on = true;
     } else {
       on = cell_is_on(M, lf, ci);
     }
-  } else if (ESZ > 0 && out_vals) {
-    for (int k = 0; k < ESZ; k++) d[k] = 0;
   }
+  // what an off cell holds is not shown: this library keeps it at T{}, but a caller's kernel
+  // may turn cells off in the masks of bxg_grid_device_view
+  if (!on) v = 0;
+  if (ESZ > 0 && out_vals) copy_val<ESZ>(out_vals + static_cast<size_t>(i) * ESZ, vp);
   if (found) found[i] = on;
 }
 
