@@ -420,8 +420,9 @@ extern "C" int bxg_grid_deserialize(bxg_grid g, const void* data, size_t n) {
   if (!plain || leaves.size() >= 0x7FFFFFFFu)
     return set_in_file_order(g, m, body, nroots, cells);
   cudaSetDevice(m->device);
-  int st = core_reserve(m, leaves.size(), nroots);
-  if (st) return st;
+  // room for the leaves that the grid does not have yet, at most all; what cannot be had
+  // now may not be needed, and otherwise the pools grow on demand
+  if (core_reserve(m, leaves.size(), nroots)) m->err.clear();
   BXG_CUDA(m, m->s_in.ensure(size_t(p - body)));
   BXG_CUDA(m, m->s_in2.ensure(leaves.size() * sizeof(FileLeaf)));
   BXG_CUDA(m, cudaMemcpyAsync(m->s_in.p, body, size_t(p - body), cudaMemcpyHostToDevice,

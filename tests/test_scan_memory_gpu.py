@@ -150,3 +150,18 @@ def test_a_tick_that_finds_no_memory_for_its_lists(gpu, port, alloc_limit, max_r
     tick([sphere(rng, n, 9.0) for _ in maps], max_range)
     for m, o in zip(maps, orc):
         same(m, o)
+
+
+def test_loading_over_the_same_leaves_needs_no_pool(gpu, alloc_limit):
+    """A file whose leaves the grid has is loaded without memory for other ones."""
+    rng = np.random.default_rng(9)
+    leaf = np.stack(np.meshgrid(*[np.arange(8)] * 3, indexing="ij"), -1).reshape(-1, 3) * 8
+    xyz = np.concatenate([leaf + rng.integers(0, 8, leaf.shape) for _ in range(3)])
+    xyz = np.unique(xyz, axis=0).astype(np.int32)
+    g = gpu.VoxelGrid(0.1, dtype=np.float32, config=gpu.Config(initial_leaves=700))
+    g.set_values(xyz, rng.normal(size=len(xyz)).astype(np.float32))
+    want, saved = g.dump(), g.serialize()
+    g.set_values(xyz, np.zeros(len(xyz), np.float32))
+    assert alloc_limit(1 << 20) == 0  # the pool of 700 leaves has more
+    g.deserialize(saved)
+    assert all(np.array_equal(a, b) for a, b in zip(g.dump(), want))
