@@ -384,7 +384,7 @@ class VoxelGrid(_Handle):
         out = new(None, n.value)
         self._check(self.lib.bxg_grid_serialize(self.h, type_name.encode(), out, n.value,
                                                 C.byref(n)))
-        return out
+        return out[:n.value]  # itself, unless the map has shrunk in between
 
     def deserialize(self, data: bytes):
         self._check(self.lib.bxg_grid_deserialize(self.h, data, len(data)))
