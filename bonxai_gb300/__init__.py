@@ -66,6 +66,10 @@ class Options(C.Structure):
                 ("occupancy_threshold_log", C.c_int32)]
 
 
+# PyBytes_FromStringAndSize, as a function of this module's own (one taken from C.pythonapi
+# has its types for the whole process)
+_new_bytes = C.PYFUNCTYPE(C.py_object, C.c_char_p, C.c_ssize_t)(
+    ("PyBytes_FromStringAndSize", C.pythonapi))
 _vp, _sz, _int, _dbl, _u64p = C.c_void_p, C.c_size_t, C.c_int, C.c_double, C.POINTER(C.c_uint64)
 _SIGS = {
     "bxg_config_default": (None, [_vp]),
@@ -379,9 +383,7 @@ class VoxelGrid(_Handle):
         if st not in (0, 7):
             self._check(st)
         # a bytes object of that size, filled before anyone else sees it
-        new = C.pythonapi.PyBytes_FromStringAndSize
-        new.restype, new.argtypes = C.py_object, [C.c_char_p, C.c_ssize_t]
-        out = new(None, n.value)
+        out = _new_bytes(None, n.value)
         self._check(self.lib.bxg_grid_serialize(self.h, type_name.encode(), out, n.value,
                                                 C.byref(n)))
         return out[:n.value]  # itself, unless the map has shrunk in between

@@ -29,3 +29,8 @@ def test_as_many_bytes_as_were_written():
     assert grid([10, 10]).serialize() == b"0123456789"
     assert grid([10, 4]).serialize() == b"0123"
 
+
+def test_the_interpreters_function_is_left_alone():
+    before = C.pythonapi.PyBytes_FromStringAndSize.restype
+    grid([10, 10]).serialize()
+    assert C.pythonapi.PyBytes_FromStringAndSize.restype is before is C.c_int
