@@ -553,6 +553,7 @@ struct bxg_batch_s {
   int grid = 0;          // resident blocks of the single-pass tick
   size_t grid_smem = 0;  // dynamic shared memory that was sized for
   int grid_mark = 0;     // blocks of the two-phase tick's mark phase
+  int last_grid = 0;     // of the last tick
   bool use_graph = true;
   // device buffers
   DevBuf pts, ep, tab, cast, segs, tails, roots, meta, params;
@@ -880,6 +881,7 @@ int batch_insert(bxg_batch b, const bxg_pmap* maps, size_t n_scans, const float*
   cudaEventRecord(b->ev1, b->stream);
   BB_CUDA(b, cudaStreamSynchronize(b->stream));
   b->launches++;
+  b->last_grid = mark ? b->grid_mark : b->grid;
   cudaEventElapsedTime(&b->last_ms, b->ev0, b->ev1);
   b->ticks++;
 
@@ -975,7 +977,7 @@ int bxg_batch_create(bxg_batch* out, const bxg_config* cfg_in) {
   cudaFuncSetAttribute(k_tick<32, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   cudaFuncSetAttribute(k_tick<16, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   cudaFuncSetAttribute(k_tick<8, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  b->grid_mark = b->sm_count * kMarkBlocksPerSM;
+  b->grid_mark = b->last_grid = b->sm_count * kMarkBlocksPerSM;
   cudaGetLastError();
   const size_t pbytes = 256 + kMaxTickScans * sizeof(TickScan);
   if (cudaMallocHost(reinterpret_cast<void**>(&b->h_args), pbytes) != cudaSuccess ||
@@ -1017,7 +1019,7 @@ int bxg_batch_stats(bxg_batch b, double out[8]) {
   out[1] = b->graph_ok ? 1 : 0;
   out[2] = double(b->last_retries);
   out[3] = double(b->ticks);
-  out[4] = double(b->grid ? b->grid : b->grid_mark);
+  out[4] = double(b->last_grid);
   out[5] = double(b->launches);
   out[6] = b->phase_ms[1];  // endpoints
   out[7] = b->phase_ms[2] + b->phase_ms[4];  // winners + rays
