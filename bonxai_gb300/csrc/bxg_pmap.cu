@@ -678,8 +678,12 @@ int finish_scan(bxg_pmap_s* pm, int ox, int oy, int oz, bool cast_rays, uint64_t
   if (ray_cells) *ray_cells = (include_points ? hs[S_POINTS] : 0) + hs[S_RAY_LEN];
   if (m->flags & BXG_FLAG_TIMING) {
     for (int k = 0; k < 4; k++) {
-      float ms = 0;
-      if (pm->ev[k] && pm->ev[k + 1]) cudaEventElapsedTime(&ms, pm->ev[k], pm->ev[k + 1]);
+      float ms = 0;  // a phase that never ran has no event yet
+      if (pm->ev[k] && pm->ev[k + 1] &&
+          cudaEventElapsedTime(&ms, pm->ev[k], pm->ev[k + 1]) != cudaSuccess) {
+        cudaGetLastError();
+        ms = 0;
+      }
       pm->last_times[k] = ms;
     }
   }
