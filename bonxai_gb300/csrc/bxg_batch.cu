@@ -802,10 +802,9 @@ int batch_insert(bxg_batch b, const bxg_pmap* maps, size_t n_scans, const float*
     A.root_words += cube_root_words(S.Q);
     root_room += uint64_t(S.Q.SR) * S.Q.SR * S.Q.SR;
     seg0[s] = seg_room;
-    // a segment is a ray's position (24 bits) and a number (8 bits); scans for which the
-    // lists of all scans would take more than 2 GB are walked ray by ray
+    // scans for which the lists of all scans would take more than 2 GB are walked ray by ray
     const uint64_t need = uint64_t(S.n) * max_segments(S.Q);
-    has_segs[s] = S.n <= (1u << 24) && seg_room + need <= (1u << 29);
+    has_segs[s] = S.n <= kMaxSegRays && seg_room + need <= (1u << 29);
     if (has_segs[s]) seg_room += need;
   }
   if (mark) {

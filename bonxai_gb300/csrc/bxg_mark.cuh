@@ -120,17 +120,21 @@ constexpr uint32_t kNearCells = 8 * kNearNB + 1;
 constexpr uint32_t kNearW = 2 * kNearNB + 1;     // words of 8 x 4 cells: 7 x 14 x 56
 constexpr uint32_t kNearWords = kNearW * 2 * kNearW * 8 * kNearW;
 constexpr uint32_t kSegCells = 32;
+constexpr uint32_t kSegBits = 5;                 // of a segment's number, beside its ray's
+constexpr uint32_t kMaxSegRays = 1u << (32 - kSegBits);
 constexpr uint32_t kMarkMaxRay = 32768;          // longer rays are walked on the tree (k_tail)
 constexpr uint32_t kFmaMaxRay = 2047;
 constexpr int kMaxCubeHalf = 24;                 // roots on each side: bit addresses in 32 bits
 constexpr int kOpenCubeHalf = 16;                // of a scan whose rays may be of any length
+static_assert((32 * kMaxCubeHalf + 1 - kNearCells + kSegCells - 1) / kSegCells <= 1u << kSegBits,
+              "segments of the longest ray");
 constexpr uint32_t kRootFlagWords =
     ((2 * kMaxCubeHalf + 1) * (2 * kMaxCubeHalf + 1) * (2 * kMaxCubeHalf + 1) + 31) / 32;
 
 struct ScanCube {
   uint32_t* bits;   // S^3 leaf blocks of 16 words, x fastest; zero between scans
   uint32_t* roots;  // one bit per root (SR^3), set by the segments
-  uint32_t* segs;   // segments: ray << 8 | number; nullptr: rays are walked whole
+  uint32_t* segs;   // segments: ray << kSegBits | number; nullptr: rays are walked whole
   uint32_t* tails;  // rays longer than kin; nullptr: there are none
   int x0, y0, z0;   // lowest cell (multiples of 32)
   uint32_t S, SR;   // leaves, roots per side
@@ -345,7 +349,7 @@ __device__ __forceinline__ void mark_scan(const DMap& M, const ScanCube& Q,
   int4 e = make_int4(0, 0, 0, 0);
   if (s < s_end) {
     seg = segment(s);
-    e = cast[seg >> 8];
+    e = cast[seg >> kSegBits];
   }
   if (r < r_end)
     for (uint32_t t = threadIdx.x; t < kNearWords; t += kMarkThreads) S.near[t] = 0u;
@@ -373,12 +377,12 @@ __device__ __forceinline__ void mark_scan(const DMap& M, const ScanCube& Q,
   }
   while (s < s_end) {
     const MarkRay q = mark_ray(M, Q, e, ox, oy, oz);
-    const uint32_t ka = kNearCells + (seg & 255u) * kSegCells;
+    const uint32_t ka = kNearCells + (seg & ((1u << kSegBits) - 1u)) * kSegCells;
     const uint32_t kb = min(ka + kSegCells, q.m);
     s += s_step;
     if (s < s_end) {
       seg = segment(s);
-      e = cast[seg >> 8];
+      e = cast[seg >> kSegBits];
     }
     int ax, ay, az, bx, by, bz;
     if (__any_sync(0xffffffffu, q.len > kFmaMaxRay)) {
@@ -700,7 +704,7 @@ __device__ __forceinline__ void winners_block(const DMap& M, const int4* __restr
   for (uint32_t j = 0;; ++j) {
     const unsigned has = __ballot_sync(0xffffffffu, nseg > j);
     if (!has) break;
-    if (nseg > j) Q.segs[at + __popc(has & ((1u << lane) - 1u))] = (ray << 8) | j;
+    if (nseg > j) Q.segs[at + __popc(has & ((1u << lane) - 1u))] = (ray << kSegBits) | j;
     at += __popc(has);
   }
 }
