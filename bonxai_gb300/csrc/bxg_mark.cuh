@@ -727,11 +727,15 @@ __device__ __forceinline__ void endpoint_enter(const DMap& M, int4& e, uint32_t 
 
 // The parts of rays that the cube does not hold (cells k >= kin; all cells of a
 // ray of kMarkMaxRay cells or more), walked on the tree. A warp takes a piece of a
-// ray, 1 / kTailPieces of it and at least two steps of 32 cells: a walk is a
-// chain of dependent loads, about 4 us a step, and the rays that go far are few
-// (29 k points at 0.05 m with returns to 100 m: 16 us; with eight rays per warp and
-// pieces of 256 cells 125 us; the whole scan walked by k_rays 330 us, against 17
-// for k_mark, 25 for k_apply_rays and this).
+// ray, of at least two steps of 32 cells: a walk is a chain of dependent loads, about 4 us a
+// step, and the rays that go far are few (29 k points at 0.05 m with returns to 100 m, in 32
+// pieces: 16 us; with eight rays per warp and pieces of 256 cells 125 us; the whole scan
+// walked by k_rays 330 us, against 17 for k_mark, 25 for k_apply_rays and this). Where they
+// are many a piece costs more than it gives -- finding its place divides in 64 bits, and
+// most pieces of a ray that is not much longer than the cube are empty: about four pieces
+// per warp then, down to whole rays (whole scans of 131 k points whose rays all have 800
+// cells: 0.83 ms, 2.8 in 32 pieces, 0.98 walked by k_rays; of 30 k with a fifth of such
+// rays 163 us, 234, 197; of 2 k with rays of 3000-8000 cells 365, 373, 620).
 constexpr uint32_t kTailPieces = 32;
 __device__ __forceinline__ void tail_rays(const DMap& M, const ScanCube& Q,
                                           const int4* __restrict__ cast, uint32_t cast_cap,
@@ -739,9 +743,11 @@ __device__ __forceinline__ void tail_rays(const DMap& M, const ScanCube& Q,
                                           int32_t u, int32_t miss, int32_t cmin,
                                           uint32_t& visited, uint32_t& updated) {
   const uint32_t n = min(ld_volatile(M.ctr + C_TAILS), cast_cap);
+  if (!n) return;
   const unsigned lane = threadIdx.x & 31;
-  for (uint64_t t = warp; t < uint64_t(n) * kTailPieces; t += n_warps) {
-    const uint32_t i = uint32_t(t / kTailPieces), j = uint32_t(t % kTailPieces);
+  const uint32_t pieces = uint32_t(max(min(4 * n_warps / n, uint64_t(kTailPieces)), uint64_t(1)));
+  for (uint64_t t = warp; t < uint64_t(n) * pieces; t += n_warps) {
+    const uint32_t i = uint32_t(t / pieces), j = uint32_t(t % pieces);
     const int4 e = cast[Q.tails[i]];
     const uint32_t m = chebyshev(ox, oy, oz, e.x, e.y, e.z);
     if (m >= kMaxRayCells) {
@@ -749,7 +755,7 @@ __device__ __forceinline__ void tail_rays(const DMap& M, const ScanCube& Q,
       continue;
     }
     const uint32_t from = m < kMarkMaxRay ? Q.kin : 0u;
-    const uint32_t piece = max(64u, (((m - from) / kTailPieces + 32u) & ~31u));
+    const uint32_t piece = max(64u, (((m - from) / pieces + 32u) & ~31u));
     if (from + j * piece < m)
       walk_ray<32>(M, e, ox, oy, oz, u, miss, cmin, lane, 0u, 0xffffffffu, visited, updated,
                    nullptr, from + j * piece, from + (j + 1) * piece);
