@@ -276,7 +276,7 @@ namespace bxg {
 // within `reach` (world units) of the origin; with `reach` infinite or above the
 // size limit, Q->open is set and the cube holds the rays' first Q->kin
 // cells. *ok = false when the scan cannot use one (other node sizes, non-finite
-// points kept, single pass asked for, no memory for it). rays: room for their
+// points kept, single pass asked for, no memory for it) or is faster without. rays: room for their
 // segments (0: none). Buffers grow here (cudaMalloc, zeroed).
 int scan_cube(bxg_pmap_s* pm, int ox, int oy, int oz, double reach, uint64_t rays, ScanCube* Q,
               bool* ok);

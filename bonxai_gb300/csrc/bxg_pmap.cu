@@ -448,6 +448,8 @@ int leaf_dir_for_scan(bxg_pmap_s* pm, int ox, int oy, int oz, LeafDir* D, size_t
 }  // namespace bxg
 
 namespace bxg {
+constexpr uint64_t kOpenRays = 65536;
+constexpr double kOpenCells = 1024.0;
 // Ray ends lie within this many cells of the origin cell (the floor of the origin and of
 // the end each move a cell by less than one).
 static double reach_cells(const MapCore* m, double reach) {
@@ -476,6 +478,16 @@ int scan_cube(bxg_pmap_s* pm, int ox, int oy, int oz, double reach, uint64_t ray
     return BXG_OK;
   int h = kOpenCubeHalf;
   if (open_reach(m, reach)) {
+    // With a range just above the largest cube, every ray without a return leaves the cube by
+    // little, and the tree is faster up to some ten thousand points (us, on the tree and
+    // with the cube: LiDAR, 800 cells at 0.2 m, 2 k points 82, 102, 8 k 97, 119, 30 k 170, 178,
+    // 131 k 235, 195; room, 1000 cells at 5 mm, 2 k 108, 212, 30 k 392, 499). Beyond, few rays
+    // are that long (LiDAR, 1200 cells at 0.05 m, 2 k 123, 115, 8 k 169, 139; 2000 cells 8 k
+    // 290, 163; no limit, returns to 100 m, 2 k 139, 80).
+    if (rays && rays < kOpenRays && reach_cells(m, reach) <= kOpenCells) {
+      *Q = ScanCube{};
+      return BXG_OK;
+    }
     Q->open = 1;
     if (core_mem_usage(m) + kOpenCubeBytes > m->budget) {
       drop_open_cube(pm);

@@ -45,3 +45,20 @@ def test_all_rays_long_no_slower_than_on_the_tree(gpu):
             t.append(time.perf_counter() - a)
     # 0.85 of it for a LiDAR's 131 k rays of 800 cells; 2.9 with 32 pieces for each ray
     assert np.median(took[0][8:]) < 1.5 * np.median(took[1][8:])
+
+
+@pytest.mark.parametrize("cells,n,on_tree", [(769, 60000, True), (1020, 2000, True),
+                                             (1100, 2000, False)])
+def test_ranges_above_the_cube(gpu, port, cells, n, on_tree):
+    """Scans of a range just above the largest cube are walked on the tree: by one kernel after
+    those of the endpoints and winners, not by three."""
+    rng = np.random.default_rng(cells)
+    m = gpu.ProbabilisticMap(RES, gpu.Config(initial_leaves=1 << 16))
+    o = port.pmap(RES)
+    for _ in range(2):
+        p = rays(rng, n, 300, 1.5 * cells)
+        before = m.last_stats()["launches"]
+        assert m.insert_point_cloud(p, np.zeros(3, np.float32), cells * RES) == \
+            o.insert(p, np.zeros(3, np.float32), cells * RES)
+    assert m.last_stats()["launches"] - before == (3 if on_tree else 5)
+    assert all(np.array_equal(a, b) for a, b in zip(m.dump(), o.dump()))
