@@ -10,12 +10,6 @@ namespace bxg {
 // ---------------------------------------------------------------------------
 // kernels
 // ---------------------------------------------------------------------------
-__global__ void k_fill_u32(uint32_t* p, uint32_t v, size_t n) {
-  for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n;
-       i += size_t(gridDim.x) * blockDim.x)
-    p[i] = v;
-}
-
 // Re-inserts the old root buckets into a larger, empty table.
 __global__ void k_rehash(const uint4* __restrict__ old_b, uint32_t old_cap, const __grid_constant__ DMap M) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -428,7 +422,6 @@ int core_sync(MapCore* m, uint32_t* err_bits_out) {
 int core_grow_for(MapCore* m, uint32_t err) {
   int st = BXG_OK;
   if (err & ERR_POOL_INNER) {
-    // the counter overshoots by the number of failed requests: a fair estimate
     st = grow_inner(m, std::max<size_t>(size_t(m->dm.icap) * 2, size_t(m->dm.icap) + 1024));
     if (st) return st;
   }
