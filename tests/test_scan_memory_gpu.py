@@ -68,6 +68,9 @@ def test_a_tick_without_a_range_limit(gpu, port):
 def test_a_server_without_a_range_limit(gpu, port):
     """The bitmaps of a server's maps are within its budget, behind the pools."""
     n, budget = 6, 400 * MB
+    first = gpu.Server([0.2])  # loads the kernels
+    first.wait_insert(first.insert(0, clouds(0, 1, 100)[0], np.zeros(3, np.float32), INF))
+    first.close()
     before = free_bytes()
     s = gpu.Server([0.2] * n, gpu.ServerConfig(pool_budget_bytes=budget))
     orc = [port.pmap(0.2) for _ in range(n)]
