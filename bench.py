@@ -23,8 +23,8 @@ Metric: ray-cell updates/s, V / t with V = points + sum of cast ray lengths
 * ``tick_ms_p50`` / ``tick_ms_p99``: latency of one batched tick call.
 * ``roofline``: the k_tick_* kernels, algorithmic bytes per tick over its event-timed
   duration, against the measured HBM copy bandwidth.
-* ``cpu_baseline``: the CPU path (the oracle restatement, timed against the
-  reference in profiles/cpu_port_vs_ref.md) on all host cores, whole maps
+* ``cpu_baseline``: the CPU path (the oracle restatement, whose timing is level
+  with the reference's) on all host cores, whole maps
   per process, one tick or more.
 
 Other workloads (``--workload``): ``lidar`` (one map, 64x2048 LiDAR scans),
@@ -787,8 +787,7 @@ def mm_cpu_baseline(n_maps, cores, seconds, max_points=None):
             "sample": f"{ticks} tick(s) of all {n_maps} maps, maps spread over {farm.cores} "
                       f"processes, {wall:.1f} s wall; single-core rate "
                       f"{V / busy:.4g} ray-cell updates/s ({busy:.1f} s of one-core work). "
-                      "The port's timing is within 10 % of the reference compiled unmodified "
-                      "(profiles/cpu_port_vs_ref.md)"}
+                      "The port's timing is within 10 % of the reference compiled unmodified"}
 
 
 def run_reference_multimap(args):

@@ -19,9 +19,10 @@
 // The grids are one or two resident waves, whatever the tick holds, so that one
 // captured graph serves ticks of any sizes. Separate launches instead of phases of one
 // persistent kernel let each have its own registers, shared memory and occupancy.
-// When a map keeps non-finite points or asks for the single-pass ray phase, the tick
-// runs as that persistent cooperative kernel (k_tick): the same phases separated by grid
-// barriers, and rays walked on the tree by groups of W lanes.
+// When a map keeps non-finite points or asks for the single-pass ray phase, or there is no
+// memory for a map's bitmap or the tick's lists, the tick runs as that persistent
+// cooperative kernel (k_tick): the same phases separated by grid barriers, and rays walked
+// on the tree by groups of W lanes.
 //
 // Each map keeps its own pools and counters; the tick touches no state shared
 // between maps except the read-only descriptors. The arithmetic is exactly that
@@ -207,7 +208,8 @@ __global__ void __launch_bounds__(256) k_tick_endpoints(const TickArgs* __restri
 }
 
 // 32 registers for eight blocks per SM: 0.33 ms for 8 M points of 64 maps (48 registers
-// and five blocks 0.48 ms: the chain of table, root, leaf and cell loads wants warps).
+// and five blocks 0.48 ms: the chain of table, root, leaf and cell loads wants warps; what
+// does not fit, 12 bytes a thread, is spilled).
 __global__ void __launch_bounds__(256, 8) k_tick_winners(const TickArgs* __restrict__ argp,
                                                       const TickScan* __restrict__ sc) {
   __shared__ WinnersShared W;
@@ -318,8 +320,9 @@ __global__ void __launch_bounds__(256) k_tick_roots(const TickArgs* __restrict__
 }
 
 // 64 maps, 318 M updated cells: 1.28 ms (1.5 ms as a phase of the persistent kernel, eight
-// lanes per leaf), bound by the DRAM sectors of the cells; eight blocks per SM, and four
-// times as many blocks as that, to even out rows of very different work (one such wave: 1.32 ms).
+// lanes per leaf), bound by the DRAM sectors of the cells; eight blocks per SM (32 registers, 88 bytes
+// a thread spilled), and four times as many blocks as that, to even out rows of very
+// different work (one such wave: 1.32 ms).
 __global__ void __launch_bounds__(256, 8) k_tick_apply(const TickArgs* __restrict__ argp,
                                                        const TickScan* __restrict__ sc) {
   __shared__ ApplyShared W;

@@ -88,9 +88,9 @@ __device__ __forceinline__ uint32_t apply_leaf_slot(const DMap& M, int lx, int l
 //
 // and floor(fma(k, fl(d fl(1/m)), 1/2 + sign(d)/(4m))) is exactly that for k < 801
 // and m <= 2047: the values (2 k |d| + m) / (2 m) are multiples of 1/(2m), so adding
-// half of that keeps each 1/(4m) >= 1.2e-4 from the next integer, and the
-// error (k 2^-24 of the slope, 2^-15 of the rounded sum, 2^-25 of the offset)
-// stays below 8e-5; for d < 0 the value is 1 more than the floor of k d/m - 1/2 -
+// half of that keeps each 1/(4m) >= 1.22e-4 from the next integer, and the
+// error (1.5 k 2^-24 of the slope, which is rounded twice, 2^-15 of the rounded sum, 2^-25 of
+// the offset) stays below 1.03e-4; for d < 0 the value is 1 more than the floor of k d/m - 1/2 -
 // 1/(4m), which is never an integer. (All d, m and k of the range: compared on a CPU.)
 // Added to 2^23 + the origin's cell and rounded down, the float's low bits are the
 // cell's coordinate: no conversion, sign or origin is left to apply, and the exponent's

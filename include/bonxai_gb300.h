@@ -52,7 +52,9 @@ typedef enum {
 
 /* Pool/stream configuration; zero-initialise and set what you need. */
 typedef struct {
-  size_t pool_budget_bytes; /* max device bytes for hash+inner+leaf pools; 0 = 16 GiB */
+  size_t pool_budget_bytes; /* max device bytes for hash+inner+leaf pools, and behind them
+                             * for the ray bitmap (147 MB) of scans without a range limit,
+                             * which do without it when it does not fit; 0 = 16 GiB */
   uint32_t initial_leaves;  /* leaf slots allocated up front; 0 = 4096 */
   uint32_t initial_inners;  /* inner slots allocated up front; 0 = 1024 */
   uint32_t hash_buckets;    /* root hash buckets (power of two); 0 = 4096 */
@@ -385,7 +387,8 @@ int bxg_batch_phase_ms(bxg_batch b, double out[6]);
 typedef struct bxg_server_s* bxg_server;
 
 typedef struct {
-  size_t pool_budget_bytes;      /* across all maps' node pools; 0 = 40 GiB */
+  size_t pool_budget_bytes;      /* across all maps' node pools (and, behind them, ray
+                                  * bitmaps, as in bxg_config); 0 = 40 GiB */
   uint32_t max_scans_per_tick;   /* insert slots per tick (<= 128); 0 = 128 */
   uint64_t max_points_per_tick;  /* 0 = 64 Mi points */
   uint64_t max_lookups_per_tick; /* 0 = 64 Mi coordinates */

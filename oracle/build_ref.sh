@@ -3,8 +3,8 @@
 # bonxai_map/src/probabilistic_map.cpp, compiled unmodified from where they lie,
 # behind the C API in oracle/oracle_api.h (test infrastructure only).
 #
-# Only this container has the reference sources; the GPU machine uses the golden
-# fixtures under tests/golden/ and the restatement in oracle/bonxai_oracle.cpp.
+# Where the reference sources are not mounted, the golden fixtures under
+# tests/golden/ and the restatement in oracle/bonxai_oracle.cpp take its place.
 # Usage: oracle/build_ref.sh [reference_root]   (default /root/reference)
 set -euo pipefail
 HERE="$(cd "$(dirname "$0")" && pwd)"
