@@ -212,10 +212,11 @@ __global__ void __launch_bounds__(kMarkThreads, kMarkBlocksPerSM) k_mark(
   // 22.8; depth, 70 k: 63.0, 59.4, 59.0). On both sides of the line, mark and apply with one
   // ray and two: LiDAR, 4.7 k rays 24.5, 26.6, 14 k 31.4, 32.7, 29 k 42.3, 42.0; room at 2 cm
   // 8.6 k 32.5, 34.8, 18 k 36.8, 38.2, 35 k 48.8, 45.8; depth 8.2 k 25.9, 27.0, 16 k 29.0,
-  // 28.7: one is a little faster up to about 20 k, also above the line. The segments start at the blocks after them: no
-  // block of a small scan has both (2k points: 9.5 us, 14.5 with both in the first blocks).
-  // A block takes 256 segments side by side: warps that take them 32 by 32 in turn over
-  // the grid share fewer words (2k points 13.1 us against 8.5, LiDAR 28.4 against 24.1).
+  // 28.7: one is a little faster up to about 20 k, also above the line.
+  // The segments start at the blocks after them: no block of a small scan has both (2k points:
+  // 9.5 us, 14.5 with both in the first blocks). A block takes 256 segments side by side:
+  // warps that take them 32 by 32 in turn over the grid share fewer words (2k points 13.1 us
+  // against 8.5, LiDAR 28.4 against 24.1).
   const uint32_t per = n_cast > 8192u ? 2 * kMarkThreads : kMarkThreads;
   const uint32_t near_blocks = min((n_cast + per - 1u) / per, gridDim.x);
   const uint32_t v = (blockIdx.x + gridDim.x - near_blocks) % gridDim.x;
